@@ -237,9 +237,9 @@ int moe_speculative_verify(moe_sampler* sampler, void* stream, const void* targe
 
 /* moe_speculative_verify for `sessions` Sessions in one call: the scheduler's
  * batch of Sessions that all verify `draft_count` proposals this step.  One
- * sampler launch covers every target position, one every draft position, and
- * one verification kernel walks the Sessions side by side (one CTA each); each
- * Session's outcome is what moe_speculative_verify gives for it alone.
+ * sampler launch covers every target and draft position, and one verification
+ * kernel walks the Sessions side by side (one CTA each); each Session's outcome
+ * is what moe_speculative_verify gives for it alone.
  *
  * target_logits   device, [sessions x (draft_count + 1) x row_stride], Session-major
  * draft_logits    device, [sessions x draft_count x row_stride]

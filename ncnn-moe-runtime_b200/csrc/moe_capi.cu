@@ -507,7 +507,7 @@ int moe_speculative_verify_batch(moe_sampler* sampler, void* stream_handle, cons
     }
     kept_stride = (kept_stride + 3u) & ~3u;
     const size_t list_entries = static_cast<size_t>(rows) * kept_stride;
-    const size_t dense_entries = static_cast<size_t>(sessions) * vocab;
+    const size_t dense_entries = kept_stride > MOE_SPECULATIVE_SHORT_LIST ? static_cast<size_t>(sessions) * vocab : 0;
     if (list_entries > sampler->spec_list_capacity || rows > sampler->spec_row_capacity || dense_entries > sampler->spec_dense_capacity)
     {
         // work queued on other streams may still read the old buffers
@@ -554,30 +554,28 @@ int moe_speculative_verify_batch(moe_sampler* sampler, void* stream_handle, cons
     // which the Session would draw with its uniform number draft_count of this step
     args.step_offset = draft_count;
     args.large_top_k = sampler->resident_large_top_k;
-    for (int side = 0; side < 2; ++side)
+    // target and draft positions are one batch of two logit matrices: 32 Sessions with 4 proposals are 288
+    // rows, one launch of 288 CTAs on 296 slots, where a launch per matrix left 136 and 168 slots idle
+    args.logits = target_logits;
+    args.logits_second = draft_rows > 0 ? draft_logits : nullptr;
+    args.second_begin = target_rows;
+    args.rows = rows;
+    args.params = sampler->params_dev;
+    args.token_id = sampler->spec_token;
+    args.probability = sampler->spec_probability;
+    args.row_flags = sampler->spec_flags;
+    args.row_status = sampler->spec_status;
+    args.kept_token = sampler->spec_kept_token;
+    args.kept_probability = sampler->spec_kept_probability;
+    args.kept_count = sampler->spec_kept_count;
+    args.kept_stride = kept_stride;
+    const uint32_t splits = pick_splits(sampler, rows, vocab, dtype, args.large_top_k);
+    MOE_CUDA_CHECK(sampler, launch_sample_rows(args, sampler->ws, splits, stream));
+    if (sampler->resident_needs_exact)
     {
-        const uint32_t first = side == 0 ? 0u : target_rows;
-        args.logits = side == 0 ? target_logits : draft_logits;
-        args.rows = side == 0 ? target_rows : draft_rows;
-        if (args.rows == 0)
-            continue;
-        args.params = sampler->params_dev + first;
-        args.token_id = sampler->spec_token + first;
-        args.probability = sampler->spec_probability + first;
-        args.row_flags = sampler->spec_flags + first;
-        args.row_status = sampler->spec_status + first;
-        args.kept_token = sampler->spec_kept_token + static_cast<size_t>(first) * kept_stride;
-        args.kept_probability = sampler->spec_kept_probability + static_cast<size_t>(first) * kept_stride;
-        args.kept_count = sampler->spec_kept_count + first;
-        args.kept_stride = kept_stride;
-        const uint32_t splits = pick_splits(sampler, args.rows, vocab, dtype, args.large_top_k);
-        MOE_CUDA_CHECK(sampler, launch_sample_rows(args, sampler->ws, splits, stream));
-        if (sampler->resident_needs_exact)
-        {
-            if (int status = ensure_exact_scratch(sampler, stream))
-                return status;
-            MOE_CUDA_CHECK(sampler, launch_sample_exact(args, sampler->ws, stream));
-        }
+        if (int status = ensure_exact_scratch(sampler, stream))
+            return status;
+        MOE_CUDA_CHECK(sampler, launch_sample_exact(args, sampler->ws, stream));
     }
     SpeculativeArgs verify = {};
     verify.sessions = sessions;

@@ -205,6 +205,15 @@ struct LogitTraits<__nv_bfloat16>
     }
 };
 
+// First logit of a row of a (possibly two-part) batch.
+template<typename T, typename Args>
+__device__ __forceinline__ const T* row_logits(const Args& a, uint32_t row)
+{
+    if (a.logits_second != nullptr && row >= a.second_begin)
+        return static_cast<const T*>(a.logits_second) + static_cast<size_t>(row - a.second_begin) * a.row_stride;
+    return static_cast<const T*>(a.logits) + static_cast<size_t>(row) * a.row_stride;
+}
+
 // ---- warp / block reductions ------------------------------------------------------
 __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v)
 {

@@ -12,6 +12,8 @@
 // largest top_k the small-buffer kernel instantiation serves (the 4 * k + 64 records a slice expects above its sampled
 // threshold must fit the 2048-record buffer with room for their spread)
 #define MOE_SAMPLER_TOPK_SMALL_MAX 448u
+// kept lists up to this length are verified in shared memory; longer ones need the dense residual scratch
+#define MOE_SPECULATIVE_SHORT_LIST 1024u
 // entries of the router's [expert][block] count table (expert_count * blocks of the select kernel never exceeds it)
 #define MOE_ROUTER_BLOCK_TABLE_ENTRIES 262144u
 
@@ -43,6 +45,9 @@ struct Workspace
 struct SampleArgs
 {
     const void* logits;
+    // a second logit matrix of the same stride that holds the rows from second_begin on (null: all rows are in `logits`)
+    const void* logits_second;
+    uint32_t second_begin;
     int dtype;
     uint32_t rows;
     uint32_t vocab;

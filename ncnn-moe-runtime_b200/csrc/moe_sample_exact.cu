@@ -807,7 +807,7 @@ __device__ bool exact_row_bf16_runs(const SampleArgs& a, uint32_t row, const moe
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
-    const uint16_t* bits = reinterpret_cast<const uint16_t*>(a.logits) + static_cast<size_t>(row) * a.row_stride;
+    const uint16_t* bits = row_logits<uint16_t>(a, row);
     const uint32_t vocab = a.vocab;
     out = RowOutcome{MOE_ROW_OK, -1, 0.0f, 0u, false};
     if (a.kept_count != nullptr || (a.topk_index != nullptr && p.top_k > 0 && p.top_k <= MOE_SAMPLER_TOPK_FAST_MAX))
@@ -1193,7 +1193,7 @@ __device__ void exact_row(const SampleArgs& a, uint32_t row, uint32_t* slot_keys
     const int lane = tid & 31;
     const int warp = tid >> 5;
     const moe_row_params p = a.params[row];
-    const T* row_pointer = static_cast<const T*>(a.logits) + static_cast<size_t>(row) * a.row_stride;
+    const T* row_pointer = row_logits<T>(a, row);
 
     // the slot holds two buffers of slot_stride 64-bit items; the sort ping-pongs between them
     uint64_t* items[2] = {reinterpret_cast<uint64_t*>(slot_keys), reinterpret_cast<uint64_t*>(slot_keys) + slot_stride};

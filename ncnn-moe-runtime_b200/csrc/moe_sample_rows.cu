@@ -1482,7 +1482,7 @@ __global__ void __launch_bounds__(kThreads, MOE_ROW_MIN_CTAS) sample_rows_kernel
         grid_dependency_release();
 
     // ---- the slice of this CTA, and its first bytes on request at once -----------
-    const T* row_pointer = static_cast<const T*>(a.logits) + static_cast<size_t>(row) * a.row_stride;
+    const T* row_pointer = row_logits<T>(a, row);
     const uint32_t vocab = a.vocab;
     // the row body is walked in 16-byte vectors from the first 32-byte boundary;
     // `groups` of kThreads vectors (or of one ring chunk of every lane's size if

@@ -23,11 +23,20 @@ namespace {
 
 constexpr int kVerifyThreads = 1024;
 constexpr int kVerifyWarps = kVerifyThreads / 32;
+// Kept lists up to this length (every Session has a Top-K up to it) are looked up by one warp each and
+// their residual is built in shared memory; longer ones (rows without Top-K) take the whole block and a
+// dense vector over the vocabulary.
+constexpr uint32_t kShortList = MOE_SPECULATIVE_SHORT_LIST;
 
 struct VerifyShared
 {
     SeqShared<kVerifyThreads> seq;
     float found[2];
+    float found_all[2 * MOE_SPECULATIVE_MAX_DRAFT]; // short lists: the proposal's probability, target then draft of each position
+    int32_t list_token[2][kShortList];              // short lists: the rejected position's target and draft candidates
+    float list_value[2][kShortList];
+    float residual[kShortList];                     // ... and its residual in token-id order
+    int32_t residual_id[kShortList];
     uint32_t warp_count[kVerifyWarps];
     uint32_t cursor;
     uint32_t decision; // 0 accepted, 1 rejected, 2 error
@@ -68,6 +77,30 @@ __global__ void __launch_bounds__(kVerifyThreads, 1) speculative_verify_kernel(c
     float* const residual_value = s.residual_value + static_cast<size_t>(session) * s.vocab;
     const bool greedy = p.temperature == 0.0f;
 
+    const bool short_lists = s.kept_stride <= kShortList;
+    if (short_lists && !greedy)
+    {
+        // What the walk may look up, all positions at once: one warp per list.  The walk below then costs
+        // no memory latency per position (it used to take two dependent list scans and four barriers each).
+        for (uint32_t pair = warp; pair < 2u * n; pair += kVerifyWarps)
+        {
+            const uint32_t row = (pair & 1u) == 0u ? target_first + (pair >> 1) : draft_first + (pair >> 1);
+            const int32_t token = proposed_tokens[pair >> 1];
+            const uint32_t count = min(s.kept_count[row], s.kept_stride);
+            const int32_t* tokens = s.kept_token + static_cast<size_t>(row) * s.kept_stride;
+            const float* probabilities = s.kept_probability + static_cast<size_t>(row) * s.kept_stride;
+            float found = 0.0f; // candidate_probability (session.cpp:138-148): 0 if absent
+            for (uint32_t i = lane; i < count; i += 32)
+                if (tokens[i] == token)
+                    found = probabilities[i];
+            const unsigned holder = __ballot_sync(kFullMask, found != 0.0f); // token ids are unique in a list
+            found = __shfl_sync(kFullMask, found, holder != 0u ? __ffs(holder) - 1 : 0);
+            if (lane == 0)
+                sh.found_all[pair] = found;
+        }
+        __syncthreads();
+    }
+
     uint32_t accepted = 0;
     uint32_t used = 0;
     int32_t status = MOE_ROW_OK;
@@ -97,10 +130,19 @@ __global__ void __launch_bounds__(kVerifyThreads, 1) speculative_verify_kernel(c
                 break;
             }
             const size_t stride = s.kept_stride;
-            const float target_probability = list_probability(s.kept_token + target_row * stride, s.kept_probability + target_row * stride,
-                                                              min(s.kept_count[target_row], s.kept_stride), proposed, &sh.found[0]);
-            const float draft_probability = list_probability(s.kept_token + draft_row * stride, s.kept_probability + draft_row * stride,
-                                                             min(s.kept_count[draft_row], s.kept_stride), proposed, &sh.found[1]);
+            float target_probability, draft_probability;
+            if (short_lists)
+            {
+                target_probability = sh.found_all[2u * accepted];
+                draft_probability = sh.found_all[2u * accepted + 1u];
+            }
+            else
+            {
+                target_probability = list_probability(s.kept_token + target_row * stride, s.kept_probability + target_row * stride,
+                                                      min(s.kept_count[target_row], s.kept_stride), proposed, &sh.found[0]);
+                draft_probability = list_probability(s.kept_token + draft_row * stride, s.kept_probability + draft_row * stride,
+                                                     min(s.kept_count[draft_row], s.kept_stride), proposed, &sh.found[1]);
+            }
             if (!(draft_probability > 0.0f))
             {
                 status = MOE_ROW_DRAFT_ZERO_PROBABILITY; // session.cpp:813-821
@@ -135,50 +177,108 @@ __global__ void __launch_bounds__(kVerifyThreads, 1) speculative_verify_kernel(c
         const float* draft_probability = s.kept_probability + draft_row * stride;
         const uint32_t target_count = min(s.kept_count[target_row], s.kept_stride);
         const uint32_t draft_count = min(s.kept_count[draft_row], s.kept_stride);
-        for (uint32_t i = tid; i < s.vocab; i += kVerifyThreads)
-            dense[i] = 0.0f;
-        __syncthreads();
-        for (uint32_t i = tid; i < target_count; i += kVerifyThreads)
-            dense[target_token[i]] = target_probability[i];
-        __syncthreads();
-        for (uint32_t i = tid; i < draft_count; i += kVerifyThreads)
+        const float* residual = residual_value;
+        const int32_t* residual_ids = residual_token;
+        if (short_lists)
         {
-            const int32_t id = draft_token[i];
-            const float reduced = __fsub_rn(dense[id], draft_probability[i]);
-            dense[id] = reduced > 0.0f ? reduced : 0.0f; // std::max(0.0f, ...)
-        }
-        if (tid == 0)
-            sh.cursor = 0;
-        __syncthreads();
-        // positive entries in token-id order
-        for (uint32_t base = 0; base < s.vocab; base += kVerifyThreads)
-        {
-            const uint32_t id = base + tid;
-            const float value = id < s.vocab ? dense[id] : 0.0f;
-            const bool positive = value > 0.0f;
-            const unsigned voters = __ballot_sync(kFullMask, positive);
-            if (lane == 0)
-                sh.warp_count[warp] = __popc(voters);
+            // max(0, target - draft) is only positive on target candidates: one thread per candidate finds the
+            // draft's probability of its token and its place among the positive ones by token id, in shared memory
+            // (a dense vector over the vocabulary cost three passes of vocab * 4 bytes by one CTA: 190 us at 201088)
+            residual = sh.residual;
+            residual_ids = sh.residual_id;
+            static_assert(kShortList <= kVerifyThreads, "one thread per candidate");
+            if (static_cast<uint32_t>(tid) < target_count)
+            {
+                sh.list_token[0][tid] = target_token[tid];
+                sh.list_value[0][tid] = target_probability[tid];
+            }
+            if (static_cast<uint32_t>(tid) < draft_count)
+            {
+                sh.list_token[1][tid] = draft_token[tid];
+                sh.list_value[1][tid] = draft_probability[tid];
+            }
+            if (tid == 0)
+                sh.cursor = 0;
             __syncthreads();
-            uint32_t before = sh.cursor;
-            for (int w = 0; w < warp; ++w)
-                before += sh.warp_count[w];
+            float value = 0.0f;
+            int32_t id = 0;
+            if (static_cast<uint32_t>(tid) < target_count)
+            {
+                id = sh.list_token[0][tid];
+                value = sh.list_value[0][tid];
+                for (uint32_t i = 0; i < draft_count; ++i)
+                    if (sh.list_token[1][i] == id)
+                    {
+                        const float reduced = __fsub_rn(value, sh.list_value[1][i]);
+                        value = reduced > 0.0f ? reduced : 0.0f; // std::max(0.0f, ...)
+                        break;
+                    }
+            }
+            const bool positive = value > 0.0f;
+            __syncthreads();
+            if (static_cast<uint32_t>(tid) < target_count)
+                sh.list_value[0][tid] = value;
+            const unsigned voters = __ballot_sync(kFullMask, positive);
+            if (lane == 0 && voters != 0u)
+                atomicAdd(&sh.cursor, static_cast<uint32_t>(__popc(voters)));
+            __syncthreads();
             if (positive)
             {
-                const uint32_t slot = before + __popc(voters & ((1u << lane) - 1u));
-                residual_token[slot] = static_cast<int32_t>(id);
-                residual_value[slot] = value;
+                uint32_t place = 0;
+                for (uint32_t i = 0; i < target_count; ++i)
+                    place += (sh.list_value[0][i] > 0.0f && sh.list_token[0][i] < id) ? 1u : 0u;
+                sh.residual[place] = value;
+                sh.residual_id[place] = id;
             }
-            __syncthreads();
-            if (tid == kVerifyThreads - 1)
-                sh.cursor = before + __popc(voters);
-            __syncthreads();
         }
+        else
+        {
+            for (uint32_t i = tid; i < s.vocab; i += kVerifyThreads)
+                dense[i] = 0.0f;
+            __syncthreads();
+            for (uint32_t i = tid; i < target_count; i += kVerifyThreads)
+                dense[target_token[i]] = target_probability[i];
+            __syncthreads();
+            for (uint32_t i = tid; i < draft_count; i += kVerifyThreads)
+            {
+                const int32_t id = draft_token[i];
+                const float reduced = __fsub_rn(dense[id], draft_probability[i]);
+                dense[id] = reduced > 0.0f ? reduced : 0.0f; // std::max(0.0f, ...)
+            }
+            if (tid == 0)
+                sh.cursor = 0;
+            __syncthreads();
+            // positive entries in token-id order
+            for (uint32_t base = 0; base < s.vocab; base += kVerifyThreads)
+            {
+                const uint32_t id = base + tid;
+                const float value = id < s.vocab ? dense[id] : 0.0f;
+                const bool positive = value > 0.0f;
+                const unsigned voters = __ballot_sync(kFullMask, positive);
+                if (lane == 0)
+                    sh.warp_count[warp] = __popc(voters);
+                __syncthreads();
+                uint32_t before = sh.cursor;
+                for (int w = 0; w < warp; ++w)
+                    before += sh.warp_count[w];
+                if (positive)
+                {
+                    const uint32_t slot = before + __popc(voters & ((1u << lane) - 1u));
+                    residual_token[slot] = static_cast<int32_t>(id);
+                    residual_value[slot] = value;
+                }
+                __syncthreads();
+                if (tid == kVerifyThreads - 1)
+                    sh.cursor = before + __popc(voters);
+                __syncthreads();
+            }
+        }
+        __syncthreads();
         const uint32_t positives = sh.cursor;
         __syncthreads();
         // std::accumulate over the dense vector (session.cpp:171-176) = the positive entries added in token-id
         // order; replayed bit-exactly by the whole block (the entries are not sorted by value)
-        const float normalizer = block_sequential_sum<kVerifyThreads, 8, false>(residual_value, positives, kSeqSumOnly, 0.0f, sh.seq).acc;
+        const float normalizer = block_sequential_sum<kVerifyThreads, 8, false>(residual, positives, kSeqSumOnly, 0.0f, sh.seq).acc;
         if (positives == 0 || !(normalizer - normalizer == 0.0f) || normalizer <= 0.0f)
         {
             if (tid == 0)
@@ -192,14 +292,14 @@ __global__ void __launch_bounds__(kVerifyThreads, 1) speculative_verify_kernel(c
         {
             const float uniform = philox_uniform(p.seed, p.row_id, p.step + used);
             const float sample_value = __fmul_rn(uniform, normalizer); // uniform_real_distribution<float>(0, normalizer)
-            const SeqResult draw = block_sequential_sum<kVerifyThreads, 8, false>(residual_value, positives, kSeqExceedBound, sample_value, sh.seq);
+            const SeqResult draw = block_sequential_sum<kVerifyThreads, 8, false>(residual, positives, kSeqExceedBound, sample_value, sh.seq);
             // session.cpp:189-197: the last positive entry if the sum never passes the draw
             const uint32_t chosen = draw.stopped ? draw.taken - 1u : positives - 1u;
             if (tid == 0)
             {
                 sh.decision = 0;
-                sh.cursor = static_cast<uint32_t>(residual_token[chosen]);
-                sh.found[0] = __fdiv_rn(residual_value[chosen], normalizer);
+                sh.cursor = static_cast<uint32_t>(residual_ids[chosen]);
+                sh.found[0] = __fdiv_rn(residual[chosen], normalizer);
             }
         }
         __syncthreads();

@@ -168,3 +168,21 @@ def test_batch_of_sessions_equals_each_session_alone(pkg, parity, torch_cuda):
                                              np.zeros(sessions + 1, dtype=pkg.ROW_PARAMS_DTYPE))
     finally:
         sampler.close()
+
+
+@pytest.mark.parametrize("top_k", [1, 31, 33, 1000, 1024, 1025])
+def test_short_and_long_candidate_lists(pkg, parity, torch_cuda, top_k):
+    """Kept lists of up to 1024 candidates are verified in shared memory, one thread per candidate; longer ones over a dense
+    vector: both sides of that line, and lists around one warp, against the reference loop (a poor draft model: rejections)."""
+    rng = np.random.default_rng([78, top_k])
+    vocab, draft_count = 5003, 4
+    sampler = pkg.Sampler(max_rows=2 * draft_count + 1, max_vocab=vocab)
+    rejected = 0
+    try:
+        for case in range(6):
+            target, draft, proposed = _case(rng, vocab, draft_count, 1.5, top_k, 1.0, 0.0, 1.5, parity.port)
+            got = _compare(pkg, sampler, torch_cuda, parity, target, draft, proposed, (1.5, top_k, 1.0, 0.0), seed=21, row_id=case, step=case)
+            rejected += int(got["status"] == 0 and got["accepted"] < draft_count)
+    finally:
+        sampler.close()
+    assert rejected > 0
