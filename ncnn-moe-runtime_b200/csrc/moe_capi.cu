@@ -33,8 +33,8 @@ struct moe_sampler
     bool overlap_launches = false;
     bool resident_has_stops = false;
 
-    // packed per-row results of moe_sample_tokens
-    moe_sampled_row* sampled_dev = nullptr;
+    // per-row records of moe_sample_tokens: page-locked host memory the kernels write through (allocated by its first call)
+    moe_sampled_row* sampled_host = nullptr;
 
     // staging for the host-buffer entry points
     void* logits_dev = nullptr;
@@ -283,7 +283,6 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
     allocate(reinterpret_cast<void**>(&sampler->probability_dev), sizeof(float) * max_rows);
     allocate(reinterpret_cast<void**>(&sampler->flags_dev), sizeof(uint32_t) * max_rows);
     allocate(reinterpret_cast<void**>(&sampler->status_dev), sizeof(int32_t) * max_rows);
-    allocate(reinterpret_cast<void**>(&sampler->sampled_dev), sizeof(moe_sampled_row) * max_rows);
     allocate(reinterpret_cast<void**>(&sampler->router_error), sizeof(unsigned long long));
     allocate(reinterpret_cast<void**>(&sampler->router_scan_done), sizeof(uint32_t));
     allocate(reinterpret_cast<void**>(&sampler->gather_status), sizeof(int32_t));
@@ -324,7 +323,7 @@ void moe_sampler_destroy(moe_sampler* sampler)
                         sampler->ws.slice_header, sampler->ws.row_arrivals, sampler->params_dev, sampler->stop_offsets_dev,
                         sampler->stop_tokens_dev, sampler->logits_dev, sampler->token_dev, sampler->probability_dev, sampler->flags_dev,
                         sampler->status_dev, sampler->topk_dev, sampler->selected_expert, sampler->selected_weight, sampler->expert_counts,
-                        sampler->sampled_dev, sampler->router_error, sampler->router_scan_done, sampler->router_block_counts, sampler->gather_status,
+                        sampler->router_error, sampler->router_scan_done, sampler->router_block_counts, sampler->gather_status,
                         sampler->router_logits_dev, sampler->router_bias_dev, sampler->router_explicit_dev,
                         sampler->router_offsets_dev, sampler->router_token_dev, sampler->router_rank_dev, sampler->router_weight_dev,
                         sampler->router_status_dev, sampler->spec_kept_token, sampler->spec_kept_probability, sampler->spec_kept_count,
@@ -333,6 +332,8 @@ void moe_sampler_destroy(moe_sampler* sampler)
     for (void* pointer : pointers)
         if (pointer != nullptr)
             cudaFree(pointer);
+    if (sampler->sampled_host != nullptr)
+        cudaFreeHost(sampler->sampled_host);
     if (sampler->stream != nullptr)
         cudaStreamDestroy(sampler->stream);
     delete sampler;
@@ -410,9 +411,14 @@ int moe_sample_batch(moe_sampler* sampler, void* stream_handle, const void* logi
     return moe_sample_batch_ex(sampler, stream_handle, logits, dtype, rows, vocab, row_stride, params, step_offset, stop_offsets, stop_tokens, &outputs);
 }
 
-int moe_sample_batch_ex(moe_sampler* sampler, void* stream_handle, const void* logits, int dtype, uint32_t rows, uint32_t vocab, size_t row_stride,
-                        const moe_row_params* params, uint64_t step_offset, const int32_t* stop_offsets, const int32_t* stop_tokens,
-                        const moe_sample_outputs* outputs)
+} // extern "C"
+
+namespace {
+
+// moe_sample_batch_ex; with `packed` the four per-row results leave as records instead of through the arrays of `outputs`
+int sample_rows(moe_sampler* sampler, void* stream_handle, const void* logits, int dtype, uint32_t rows, uint32_t vocab, size_t row_stride,
+                const moe_row_params* params, uint64_t step_offset, const int32_t* stop_offsets, const int32_t* stop_tokens,
+                const moe_sample_outputs* outputs, moe_sampled_row* packed)
 {
     if (int status = check_shape(sampler, dtype, rows, vocab, row_stride))
         return status;
@@ -426,7 +432,7 @@ int moe_sample_batch_ex(moe_sampler* sampler, void* stream_handle, const void* l
     int32_t* const row_status = outputs->row_status;
     int32_t* const topk_index = outputs->topk_index;
     const uint32_t topk_stride = outputs->topk_stride;
-    if (logits == nullptr || token_id == nullptr || probability == nullptr)
+    if (logits == nullptr || (packed == nullptr && (token_id == nullptr || probability == nullptr)))
         return fail(sampler, MOE_STATUS_INVALID_ARGUMENT, "logits, token_id and probability must not be null");
     if (outputs->kept_count == nullptr && (outputs->kept_token != nullptr || outputs->kept_probability != nullptr))
         return fail(sampler, MOE_STATUS_INVALID_ARGUMENT, "kept_token / kept_probability need kept_count");
@@ -455,6 +461,7 @@ int moe_sample_batch_ex(moe_sampler* sampler, void* stream_handle, const void* l
     args.probability = probability;
     args.row_flags = row_flags;
     args.row_status = row_status;
+    args.packed = packed;
     args.topk_index = topk_index;
     args.topk_stride = topk_index != nullptr ? topk_stride : 0;
     args.kept_token = outputs->kept_token;
@@ -472,6 +479,17 @@ int moe_sample_batch_ex(moe_sampler* sampler, void* stream_handle, const void* l
         MOE_CUDA_CHECK(sampler, launch_sample_exact(args, sampler->ws, stream));
     }
     return MOE_STATUS_OK;
+}
+
+} // namespace
+
+extern "C" {
+
+int moe_sample_batch_ex(moe_sampler* sampler, void* stream_handle, const void* logits, int dtype, uint32_t rows, uint32_t vocab, size_t row_stride,
+                        const moe_row_params* params, uint64_t step_offset, const int32_t* stop_offsets, const int32_t* stop_tokens,
+                        const moe_sample_outputs* outputs)
+{
+    return sample_rows(sampler, stream_handle, logits, dtype, rows, vocab, row_stride, params, step_offset, stop_offsets, stop_tokens, outputs, nullptr);
 }
 
 int moe_speculative_verify_batch(moe_sampler* sampler, void* stream_handle, const void* target_logits, const void* draft_logits, int dtype,
@@ -660,15 +678,19 @@ int moe_sample_tokens(moe_sampler* sampler, void* stream_handle, const void* log
     if (logits == nullptr || results == nullptr)
         return fail(sampler, MOE_STATUS_INVALID_ARGUMENT, "logits and results must not be null");
     cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
-    const int status = moe_sample_batch(sampler, stream, logits, dtype, rows, vocab, row_stride, params, step_offset, stop_offsets, stop_tokens,
-                                        sampler->token_dev, sampler->probability_dev, sampler->flags_dev, sampler->status_dev, nullptr, 0);
+    DeviceGuard guard(sampler->device);
+    if (sampler->sampled_host == nullptr)
+        MOE_CUDA_CHECK(sampler, cudaHostAlloc(reinterpret_cast<void**>(&sampler->sampled_host), sizeof(moe_sampled_row) * sampler->max_rows, cudaHostAllocMapped));
+    // The kernel that finishes a row stores its 16-byte record straight into host memory: a packing kernel and a
+    // device-to-host copy behind the sampler cost another two submissions and about 7 us per call.
+    moe_sampled_row* records = nullptr;
+    MOE_CUDA_CHECK(sampler, cudaHostGetDevicePointer(reinterpret_cast<void**>(&records), sampler->sampled_host, 0));
+    const moe_sample_outputs outputs = {};
+    const int status = sample_rows(sampler, stream, logits, dtype, rows, vocab, row_stride, params, step_offset, stop_offsets, stop_tokens, &outputs, records);
     if (status != MOE_STATUS_OK)
         return status;
-    DeviceGuard guard(sampler->device);
-    MOE_CUDA_CHECK(sampler, launch_pack_sampled_rows(sampler->token_dev, sampler->probability_dev, sampler->flags_dev, sampler->status_dev, rows,
-                                                     sampler->sampled_dev, stream));
-    MOE_CUDA_CHECK(sampler, cudaMemcpyAsync(results, sampler->sampled_dev, sizeof(moe_sampled_row) * rows, cudaMemcpyDeviceToHost, stream));
     MOE_CUDA_CHECK(sampler, cudaStreamSynchronize(stream));
+    std::memcpy(results, sampler->sampled_host, sizeof(moe_sampled_row) * rows);
     return MOE_STATUS_OK;
 }
 

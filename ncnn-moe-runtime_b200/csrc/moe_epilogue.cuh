@@ -264,6 +264,24 @@ __device__ __forceinline__ RowOutcome finish_row_warp(const uint64_t* records, u
     return out;
 }
 
+// The results of one row, by one thread.
+template<typename Args>
+__device__ __forceinline__ void write_row_result(const Args& a, uint32_t row, int32_t token, float probability, uint32_t flags, int32_t status)
+{
+    if (a.packed != nullptr)
+    {
+        // one 16-byte store: the record may lie across the host link
+        *reinterpret_cast<int4*>(a.packed + row) = make_int4(token, __float_as_int(probability), static_cast<int>(flags), status);
+        return;
+    }
+    a.token_id[row] = token;
+    a.probability[row] = probability;
+    if (a.row_flags != nullptr)
+        a.row_flags[row] = flags;
+    if (a.row_status != nullptr)
+        a.row_status[row] = status;
+}
+
 // Linear search of the row's stop list (src/engine/session.cpp:60-63).
 __device__ __forceinline__ bool is_stop_token(const int32_t* stop_offsets, const int32_t* stop_tokens, uint32_t row, int32_t token)
 {

@@ -60,6 +60,8 @@ struct SampleArgs
     float* probability;
     uint32_t* row_flags;   // may be null
     int32_t* row_status;   // may be null
+    // the four results above as one record per row instead (host-mapped memory of moe_sample_tokens); null: the arrays
+    moe_sampled_row* packed;
     int32_t* topk_index;   // may be null
     uint32_t topk_stride;
     // optional: every row's kept candidates with their renormalised probabilities
@@ -83,9 +85,6 @@ struct SampleArgs
 
 cudaError_t launch_sample_rows(const SampleArgs& args, const Workspace& ws, uint32_t splits, cudaStream_t stream);
 cudaError_t launch_sample_exact(const SampleArgs& args, const Workspace& ws, cudaStream_t stream);
-// token_id / probability / row_flags / row_status arrays -> one 16-byte record per row
-cudaError_t launch_pack_sampled_rows(const int32_t* token_id, const float* probability, const uint32_t* row_flags, const int32_t* row_status,
-                                     uint32_t rows, moe_sampled_row* packed, cudaStream_t stream);
 cudaError_t launch_merge_candidates(const uint64_t* gathered, uint32_t shards, uint32_t rows, uint32_t top_k, const moe_row_params* params,
                                     uint64_t step_offset, int32_t* token_id, float* probability, uint32_t* row_flags, int32_t* row_status,
                                     int32_t* topk_index, uint32_t topk_stride, cudaStream_t stream);

@@ -1343,12 +1343,7 @@ __device__ void exact_row(const SampleArgs& a, uint32_t row, uint32_t* slot_keys
     {
         if (out.status == MOE_ROW_OK && is_stop_token(a.stop_offsets, a.stop_tokens, row, out.token))
             out.flags |= MOE_ROW_FLAG_STOP_TOKEN;
-        a.token_id[row] = out.token;
-        a.probability[row] = out.probability;
-        if (a.row_flags != nullptr)
-            a.row_flags[row] = out.flags;
-        if (a.row_status != nullptr)
-            a.row_status[row] = out.status;
+        write_row_result(a, row, out.token, out.probability, out.flags, out.status);
     }
     __syncthreads();
 #ifdef MOE_PHASE_TIMERS

@@ -1438,12 +1438,7 @@ __device__ __forceinline__ void finish_row_block(const SampleArgs& a, RowShared&
             {
                 if (out.status == MOE_ROW_OK && is_stop_token(a.stop_offsets, a.stop_tokens, row, out.token))
                     out.flags |= MOE_ROW_FLAG_STOP_TOKEN;
-                a.token_id[row] = out.token;
-                a.probability[row] = out.probability;
-                if (a.row_flags != nullptr)
-                    a.row_flags[row] = out.flags;
-                if (a.row_status != nullptr)
-                    a.row_status[row] = out.status;
+                write_row_result(a, row, out.token, out.probability, out.flags, out.status);
             }
         }
     }
@@ -1550,12 +1545,7 @@ __global__ void __launch_bounds__(kThreads, MOE_ROW_MIN_CTAS) sample_rows_kernel
         {
             if (tid == 0)
             {
-                a.token_id[row] = -1;
-                a.probability[row] = 0.0f;
-                if (a.row_flags != nullptr)
-                    a.row_flags[row] = 0;
-                if (a.row_status != nullptr)
-                    a.row_status[row] = invalid;
+                write_row_result(a, row, -1, 0.0f, 0u, invalid);
                 if (a.kept_count != nullptr)
                     a.kept_count[row] = 0;
             }
@@ -1732,14 +1722,7 @@ __global__ void __launch_bounds__(kThreads, 2) merge_candidates_kernel(const uin
     if (invalid != MOE_ROW_OK)
     {
         if (tid == 0)
-        {
-            a.token_id[row] = -1;
-            a.probability[row] = 0.0f;
-            if (a.row_flags != nullptr)
-                a.row_flags[row] = 0;
-            if (a.row_status != nullptr)
-                a.row_status[row] = invalid;
-        }
+            write_row_result(a, row, -1, 0.0f, 0u, invalid);
         if (a.topk_index != nullptr)
             for (uint32_t i = tid; i < a.topk_stride; i += kThreads)
                 a.topk_index[static_cast<size_t>(row) * a.topk_stride + i] = -1;
@@ -1869,25 +1852,6 @@ cudaError_t launch_sample_rows(const SampleArgs& args, const Workspace& ws, uint
     if (args.dtype == MOE_DTYPE_F32)
         return launch_typed<float, false>(args, ws, splits, stages, stream);
     return launch_typed<__nv_bfloat16, false>(args, ws, splits, stages, stream);
-}
-
-namespace {
-__global__ void pack_sampled_rows_kernel(const int32_t* token_id, const float* probability, const uint32_t* row_flags, const int32_t* row_status,
-                                         uint32_t rows, moe_sampled_row* packed)
-{
-    const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row < rows)
-        packed[row] = moe_sampled_row{token_id[row], probability[row], row_flags[row], row_status[row]};
-}
-} // namespace
-
-cudaError_t launch_pack_sampled_rows(const int32_t* token_id, const float* probability, const uint32_t* row_flags, const int32_t* row_status,
-                                     uint32_t rows, moe_sampled_row* packed, cudaStream_t stream)
-{
-    if (rows == 0)
-        return cudaSuccess;
-    pack_sampled_rows_kernel<<<(rows + 255u) / 256u, 256, 0, stream>>>(token_id, probability, row_flags, row_status, rows, packed);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_merge_candidates(const uint64_t* gathered, uint32_t shards, uint32_t rows, uint32_t top_k, const moe_row_params* params,
