@@ -29,6 +29,7 @@ struct moe_sampler
     size_t stop_tokens_capacity = 0;
     uint32_t resident_rows = 0;
     bool resident_needs_exact = false;
+    uint32_t resident_untruncated_rows = 0; // rows without Top-K
     bool resident_large_top_k = false;
     bool overlap_launches = false;
     bool resident_has_stops = false;
@@ -154,6 +155,7 @@ int upload_rows(moe_sampler* sampler, cudaStream_t stream, uint32_t rows, const 
                 const int32_t* stop_tokens)
 {
     bool needs_exact = false;
+    uint32_t untruncated_rows = 0;
     bool large_top_k = false;
     for (uint32_t row = 0; row < rows; ++row)
     {
@@ -161,7 +163,10 @@ int upload_rows(moe_sampler* sampler, cudaStream_t stream, uint32_t rows, const 
         if (validate_row(p) != MOE_ROW_OK || p.temperature == 0.0f)
             continue;
         if (p.top_k == 0 || p.top_k > MOE_SAMPLER_TOPK_FAST_MAX)
+        {
             needs_exact = true;
+            untruncated_rows += p.top_k == 0 ? 1u : 0u;
+        }
         else if (p.top_k > MOE_SAMPLER_TOPK_SMALL_MAX)
             large_top_k = true;
     }
@@ -186,6 +191,7 @@ int upload_rows(moe_sampler* sampler, cudaStream_t stream, uint32_t rows, const 
     }
     sampler->resident_rows = rows;
     sampler->resident_needs_exact = needs_exact;
+    sampler->resident_untruncated_rows = untruncated_rows;
     sampler->resident_large_top_k = large_top_k;
     return MOE_STATUS_OK;
 }
@@ -200,7 +206,10 @@ int ensure_exact_scratch(moe_sampler* sampler, cudaStream_t stream)
         return MOE_STATUS_OK;
     const size_t stride = (static_cast<size_t>(ws.max_vocab) + 3u) & ~static_cast<size_t>(3u);
     MOE_CUDA_CHECK(sampler, cudaStreamSynchronize(stream));
-    MOE_CUDA_CHECK(sampler, cudaMalloc(reinterpret_cast<void**>(&ws.sort_keys), sizeof(uint32_t) * 4u * stride * ws.slots));
+    // one allocation: the sort scratch, then the clusters' items
+    const size_t sort_words = 4u * stride * ws.slots;
+    MOE_CUDA_CHECK(sampler, cudaMalloc(reinterpret_cast<void**>(&ws.sort_keys), sizeof(uint32_t) * (sort_words + 2u * (stride + 64u) * ws.slots)));
+    ws.exact_items = ws.sort_keys + sort_words;
     return MOE_STATUS_OK;
 }
 
@@ -271,7 +280,8 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
             status = cudaMalloc(pointer, bytes);
     };
     uint32_t* counters = nullptr;
-    allocate(reinterpret_cast<void**>(&counters), 3 * sizeof(uint32_t));
+    allocate(reinterpret_cast<void**>(&counters), 4 * sizeof(uint32_t));
+    allocate(reinterpret_cast<void**>(&ws.exact_deferred), sizeof(uint32_t) * max_rows);
     allocate(reinterpret_cast<void**>(&ws.exact_rows), sizeof(uint32_t) * max_rows);
     ws.slice_slots = static_cast<uint32_t>(sampler->sm_count) * 6u * 2u + 64u;
     allocate(reinterpret_cast<void**>(&ws.slice_records), sizeof(uint64_t) * MOE_SLICE_SLOT_RECORDS * ws.slice_slots);
@@ -288,7 +298,7 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
     allocate(reinterpret_cast<void**>(&sampler->gather_status), sizeof(int32_t));
     allocate(reinterpret_cast<void**>(&sampler->router_status_dev), sizeof(int32_t));
     if (status == cudaSuccess)
-        status = cudaMemset(counters, 0, 3 * sizeof(uint32_t));
+        status = cudaMemset(counters, 0, 4 * sizeof(uint32_t));
     if (status == cudaSuccess)
         status = cudaMemset(ws.row_arrivals, 0, sizeof(uint32_t) * max_rows);
     if (status == cudaSuccess)
@@ -304,6 +314,7 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
     ws.exact_count = counters;
     ws.exact_done = counters != nullptr ? counters + 1 : nullptr;
     ws.exact_next = counters != nullptr ? counters + 2 : nullptr;
+    ws.exact_deferred_count = counters != nullptr ? counters + 3 : nullptr;
     if (status != cudaSuccess)
     {
         moe_sampler_destroy(sampler);
@@ -319,7 +330,7 @@ void moe_sampler_destroy(moe_sampler* sampler)
         return;
     DeviceGuard guard(sampler->device);
     cudaDeviceSynchronize();
-    void* pointers[] = {sampler->ws.exact_count, sampler->ws.exact_rows, sampler->ws.sort_keys, sampler->ws.slice_records,
+    void* pointers[] = {sampler->ws.exact_count, sampler->ws.exact_rows, sampler->ws.sort_keys, sampler->ws.exact_deferred, sampler->ws.slice_records,
                         sampler->ws.slice_header, sampler->ws.row_arrivals, sampler->params_dev, sampler->stop_offsets_dev,
                         sampler->stop_tokens_dev, sampler->logits_dev, sampler->token_dev, sampler->probability_dev, sampler->flags_dev,
                         sampler->status_dev, sampler->topk_dev, sampler->selected_expert, sampler->selected_weight, sampler->expert_counts,
@@ -476,7 +487,7 @@ int sample_rows(moe_sampler* sampler, void* stream_handle, const void* logits, i
     {
         if (int status = ensure_exact_scratch(sampler, stream))
             return status;
-        MOE_CUDA_CHECK(sampler, launch_sample_exact(args, sampler->ws, stream));
+        MOE_CUDA_CHECK(sampler, launch_sample_exact(args, sampler->ws, sampler->resident_untruncated_rows, stream));
     }
     return MOE_STATUS_OK;
 }
@@ -593,7 +604,7 @@ int moe_speculative_verify_batch(moe_sampler* sampler, void* stream_handle, cons
     {
         if (int status = ensure_exact_scratch(sampler, stream))
             return status;
-        MOE_CUDA_CHECK(sampler, launch_sample_exact(args, sampler->ws, stream));
+        MOE_CUDA_CHECK(sampler, launch_sample_exact(args, sampler->ws, sampler->resident_untruncated_rows, stream));
     }
     SpeculativeArgs verify = {};
     verify.sessions = sessions;

@@ -28,9 +28,13 @@ struct Workspace
     uint32_t* exact_done = nullptr;    // [1] CTAs of the exact kernel that have finished
     uint32_t* exact_next = nullptr;    // [1] next entry of exact_rows nobody has taken yet
     uint32_t* exact_rows = nullptr;    // [max_rows]
+    // rows the clusters left to the one-CTA kernel of the same call (with a mark in the high bit), and their number
+    uint32_t* exact_deferred = nullptr;       // [max_rows]
+    uint32_t* exact_deferred_count = nullptr; // [1]
     // per-slot scratch of the exact kernel: (keys, index) pair 0 then pair 1,
     // each array `max_vocab` rounded up to a multiple of 4 entries
     uint32_t* sort_keys = nullptr;     // [slots][4][stride]
+    uint32_t* exact_items = nullptr;   // [slots][2][stride + 64]: numerators and value groups of the row a cluster works on
     // publication slots of the streaming kernel when a row is cut into slices:
     // one per CTA, MOE_SLICE_SLOT_RECORDS records and a 4-word header each
     uint64_t* slice_records = nullptr; // [slice_slots][MOE_SLICE_SLOT_RECORDS]
@@ -84,7 +88,9 @@ struct SampleArgs
 };
 
 cudaError_t launch_sample_rows(const SampleArgs& args, const Workspace& ws, uint32_t splits, cudaStream_t stream);
-cudaError_t launch_sample_exact(const SampleArgs& args, const Workspace& ws, cudaStream_t stream);
+// untruncated_rows: how many rows of the batch have no Top-K (clusters take those; the other rows a batch may hand
+// over have a Top-K above MOE_SAMPLER_TOPK_FAST_MAX)
+cudaError_t launch_sample_exact(const SampleArgs& args, const Workspace& ws, uint32_t untruncated_rows, cudaStream_t stream);
 cudaError_t launch_merge_candidates(const uint64_t* gathered, uint32_t shards, uint32_t rows, uint32_t top_k, const moe_row_params* params,
                                     uint64_t step_offset, int32_t* token_id, float* probability, uint32_t* row_flags, int32_t* row_status,
                                     int32_t* topk_index, uint32_t topk_stride, cudaStream_t stream);

@@ -5,13 +5,17 @@
 // The reference's result for such a row depends on the complete rank order
 // (src/engine/session.cpp:80-82) because its softmax normaliser, Top-P
 // cumulative, renormaliser and inverse CDF are all left-to-right fp32 sums in
-// that order (:92-101,119-134,434-440).  One CTA therefore builds the order of
-// all finite logits of the row with a stable least-significant-digit radix
-// sort in a per-CTA global scratch slot (L2 resident), and replays the sums over
-// it bit-exactly with a block-parallel scan (moe_seqscan.cuh).
+// that order (:92-101,119-134,434-440).  Three ways to replay them bit-exactly:
+//   * fp32 rows without Top-K: a thread-block cluster adds integer steps per value
+//     group, without any order (moe_exact_cluster.cuh);
+//   * rows of bf16 values, stored as bf16 or widened to fp32: one CTA works on the
+//     (value, count) runs of a histogram (moe_seqruns.cuh);
+//   * everything else: one CTA builds the order of all finite logits in a global
+//     scratch slot (L2 resident) and replays the sums with a block-parallel scan
+//     (moe_seqscan.cuh).
 //
-// CTAs take rows round-robin from the hand-over list; nobody waits on another
-// CTA.  The last CTA to finish clears the list for the next call.
+// CTAs and clusters take rows from the hand-over list; nobody waits on another
+// row.  The last CTA to finish clears the list for the next call.
 
 #include "moe_common.cuh"
 #include "moe_epilogue.cuh"
@@ -21,13 +25,13 @@
 
 #ifdef MOE_PHASE_TIMERS
 // Debug builds only: cycles per phase of the exact kernel, summed over rows.
-__device__ unsigned long long g_exact_cycles[16];
+__device__ unsigned long long g_exact_cycles[32];
 extern "C" void moe_debug_exact_cycles(unsigned long long* out, int reset)
 {
-    cudaMemcpyFromSymbol(out, g_exact_cycles, sizeof(unsigned long long) * 16);
+    cudaMemcpyFromSymbol(out, g_exact_cycles, sizeof(unsigned long long) * 32);
     if (reset)
     {
-        unsigned long long zeros[16] = {};
+        unsigned long long zeros[32] = {};
         cudaMemcpyToSymbol(g_exact_cycles, zeros, sizeof(zeros));
     }
 }
@@ -766,19 +770,40 @@ __device__ __forceinline__ float live_window_floor(float peak_logit, float tempe
     return __fsub_rn(__fsub_rn(peak_logit, __fmul_rn(18.2f, temperature)), __fmul_rn(9.5367431640625e-07f, fabsf(peak_logit)));
 }
 
+// Eight consecutive logits of a 16-byte aligned row as four words of two bf16 patterns.
+__device__ __forceinline__ uint4 load_patterns(const uint16_t* bits, uint32_t vector)
+{
+    return reinterpret_cast<const uint4*>(bits)[vector];
+}
+// ... of an fp32 row that holds nothing but bf16 values: the low halves are zero.
+__device__ __forceinline__ uint4 load_patterns(const float* row, uint32_t vector)
+{
+    const uint4 first = reinterpret_cast<const uint4*>(row)[2u * vector];
+    const uint4 second = reinterpret_cast<const uint4*>(row)[2u * vector + 1u];
+    return make_uint4(__byte_perm(first.x, first.y, 0x7632), __byte_perm(first.z, first.w, 0x7632), __byte_perm(second.x, second.y, 0x7632),
+                      __byte_perm(second.z, second.w, 0x7632));
+}
+__device__ __forceinline__ uint16_t pattern_at(const uint16_t* bits, uint32_t index)
+{
+    return bits[index];
+}
+__device__ __forceinline__ uint16_t pattern_at(const float* row, uint32_t index)
+{
+    return static_cast<uint16_t>(__float_as_uint(row[index]) >> 16);
+}
+
 // Calls visit(pattern) for every bf16 logit of the row, in no particular order:
-// 16-byte loads (eight logits) while the row is 16-byte aligned, two in flight per thread.
-template<typename Visit>
-__device__ __forceinline__ void for_each_bf16(const uint16_t* bits, uint32_t vocab, Visit visit)
+// 16-byte loads while the row is 16-byte aligned, two groups of eight logits in flight per thread.
+template<typename Stored, typename Visit>
+__device__ __forceinline__ void for_each_bf16(const Stored* bits, uint32_t vocab, Visit visit)
 {
     const uint32_t tid = threadIdx.x;
     if ((reinterpret_cast<uintptr_t>(bits) & 15u) != 0u)
     {
         for (uint32_t i = tid; i < vocab; i += kExactThreads)
-            visit(bits[i]);
+            visit(pattern_at(bits, i));
         return;
     }
-    const uint4* vectors = reinterpret_cast<const uint4*>(bits);
     const uint32_t vector_count = vocab / 8u;
     const auto visit_vector = [&](const uint4& v) {
         visit(static_cast<uint16_t>(v.x)); visit(static_cast<uint16_t>(v.x >> 16));
@@ -789,25 +814,27 @@ __device__ __forceinline__ void for_each_bf16(const uint16_t* bits, uint32_t voc
     uint32_t index = tid;
     for (; index + kExactThreads < vector_count; index += 2u * kExactThreads)
     {
-        const uint4 first = vectors[index];
-        const uint4 second = vectors[index + kExactThreads];
+        const uint4 first = load_patterns(bits, index);
+        const uint4 second = load_patterns(bits, index + kExactThreads);
         visit_vector(first);
         visit_vector(second);
     }
     if (index < vector_count)
-        visit_vector(vectors[index]);
+        visit_vector(load_patterns(bits, index));
     for (uint32_t i = vector_count * 8u + tid; i < vocab; i += kExactThreads)
-        visit(bits[i]);
+        visit(pattern_at(bits, i));
 }
 
 // Returns false when the row has to go through the sort path; `out` is only valid on true.
+// Stored: how the bf16 values lie in memory, as bf16 patterns (uint16_t) or widened to fp32 (float).
+template<typename Stored>
 __device__ bool exact_row_bf16_runs(const SampleArgs& a, uint32_t row, const moe_row_params& p, uint32_t* hist, uint32_t* scratch, uint32_t scratch_words,
                                     ExactShared& sh, RowOutcome& out)
 {
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
-    const uint16_t* bits = row_logits<uint16_t>(a, row);
+    const Stored* bits = row_logits<Stored>(a, row);
     const uint32_t vocab = a.vocab;
     out = RowOutcome{MOE_ROW_OK, -1, 0.0f, 0u, false};
     if (a.kept_count != nullptr || (a.topk_index != nullptr && p.top_k > 0 && p.top_k <= MOE_SAMPLER_TOPK_FAST_MAX))
@@ -1103,10 +1130,10 @@ __device__ bool exact_row_bf16_runs(const SampleArgs& a, uint32_t row, const moe
         if (at >= end)
             return 0u;
         if (aligned && at + 8u <= end)
-            return vector_mask(*reinterpret_cast<const uint4*>(bits + at));
+            return vector_mask(load_patterns(bits, at / 8u));
         uint32_t mask = 0;
         for (uint32_t j = 0; j < 8u && at + j < end; ++j)
-            mask |= matches(bits[at + j]) ? (1u << j) : 0u;
+            mask |= matches(pattern_at(bits, at + j)) ? (1u << j) : 0u;
         return mask;
     };
     const uint32_t part = ((vocab + kExactWarps - 1u) / kExactWarps + 255u) & ~255u; // whole trips of 32 vectors
@@ -1186,8 +1213,18 @@ __device__ bool exact_row_bf16_runs(const SampleArgs& a, uint32_t row, const moe
     return out.token >= 0;
 }
 
-template<typename T>
-__device__ void exact_row(const SampleArgs& a, uint32_t row, uint32_t* slot_keys, uint32_t* slot_index, uint32_t slot_stride, ExactShared& sh)
+// High bit of an entry of the deferred list: every logit of the fp32 row is a bf16 value.
+constexpr uint32_t kBf16ValuedRow = 0x80000000u;
+
+__device__ __noinline__ bool exact_row_widened_runs(const SampleArgs& a, uint32_t row, const moe_row_params& p, uint32_t* hist, uint32_t* scratch,
+                                                    uint32_t scratch_words, ExactShared& sh, RowOutcome& out)
+{
+    return exact_row_bf16_runs<float>(a, row, p, hist, scratch, scratch_words, sh, out);
+}
+
+// kWidened: the row may be marked as one of bf16 values widened to fp32.
+template<typename T, bool kWidened>
+__device__ void exact_row(const SampleArgs& a, uint32_t row, bool bf16_valued, uint32_t* slot_keys, uint32_t slot_stride, ExactShared& sh)
 {
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -1197,7 +1234,6 @@ __device__ void exact_row(const SampleArgs& a, uint32_t row, uint32_t* slot_keys
 
     // the slot holds two buffers of slot_stride 64-bit items; the sort ping-pongs between them
     uint64_t* items[2] = {reinterpret_cast<uint64_t*>(slot_keys), reinterpret_cast<uint64_t*>(slot_keys) + slot_stride};
-    (void)slot_index;
 
     MOE_EXACT_BEGIN();
     // rows that list their Top-K ids need every rank up to top_k: no filter for them
@@ -1209,11 +1245,18 @@ __device__ void exact_row(const SampleArgs& a, uint32_t row, uint32_t* slot_keys
     if constexpr (sizeof(T) == 2)
     {
         extern __shared__ __align__(16) uint32_t value_histogram[];
-        handled = exact_row_bf16_runs(a, row, p, value_histogram, slot_keys, 4u * slot_stride, sh, out);
+        handled = exact_row_bf16_runs<uint16_t>(a, row, p, value_histogram, slot_keys, 4u * slot_stride, sh, out);
         __syncthreads();
         if (handled && a.kept_count != nullptr && tid == 0)
             a.kept_count[row] = 0; // unreachable today (lists go through the sort path); kept for a consistent contract
         MOE_EXACT_MARK(6);
+    }
+    if constexpr (kWidened)
+    {
+        extern __shared__ __align__(16) uint32_t value_histogram[];
+        if (bf16_valued)
+            handled = exact_row_widened_runs(a, row, p, value_histogram, slot_keys, 4u * slot_stride, sh, out);
+        __syncthreads();
     }
     uint32_t floor_key = 0;
     bool has_pos_inf = false;
@@ -1355,11 +1398,25 @@ __device__ void exact_row(const SampleArgs& a, uint32_t row, uint32_t* slot_keys
 #endif
 }
 
-template<typename T>
+} // namespace
+
+} // namespace moe
+
+#include "moe_exact_cluster.cuh"
+
+namespace moe {
+
+namespace {
+
+// One CTA per row.  The rows are those the streaming kernel handed over, or (kDeferred) those of them that the
+// clusters left.
+template<typename T, bool kDeferred>
 __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_kernel(const SampleArgs a, Workspace ws)
 {
     __shared__ ExactShared sh;
-    const uint32_t pending = *ws.exact_count;
+    uint32_t* const count = kDeferred ? ws.exact_deferred_count : ws.exact_count;
+    const uint32_t* const entries = kDeferred ? ws.exact_deferred : ws.exact_rows;
+    const uint32_t pending = *count;
     const uint32_t slot_stride = (ws.max_vocab + 3u) & ~3u;
     uint32_t* slot_keys = ws.sort_keys + static_cast<size_t>(blockIdx.x) * 4u * slot_stride;
     // rows cost from a few to several hundred microseconds: a CTA takes the next one when it is free
@@ -1372,7 +1429,8 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_kernel(const Sa
         __syncthreads();
         if (entry >= pending)
             break;
-        exact_row<T>(a, ws.exact_rows[entry], slot_keys, nullptr, slot_stride, sh);
+        const uint32_t taken = entries[entry];
+        exact_row<T, kDeferred>(a, kDeferred ? taken & ~kBf16ValuedRow : taken, kDeferred && (taken & kBf16ValuedRow) != 0u, slot_keys, slot_stride, sh);
     }
     __syncthreads();
     if (threadIdx.x == 0)
@@ -1380,7 +1438,7 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_kernel(const Sa
         __threadfence();
         if (atomicAdd(ws.exact_done, 1u) == gridDim.x - 1)
         {
-            *ws.exact_count = 0; // every CTA has read it: ready for the next call
+            *count = 0; // every CTA has read it: ready for the next call
             *ws.exact_done = 0;
             *ws.exact_next = 0;
             __threadfence();
@@ -1390,26 +1448,37 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_kernel(const Sa
 
 } // namespace
 
-cudaError_t launch_sample_exact(const SampleArgs& args, const Workspace& ws, cudaStream_t stream)
+cudaError_t launch_sample_exact(const SampleArgs& args, const Workspace& ws, uint32_t untruncated_rows, cudaStream_t stream)
 {
     if (args.rows == 0 || ws.slots == 0)
         return cudaSuccess;
     const uint32_t grid = ws.slots < args.rows ? ws.slots : args.rows;
-    if (args.dtype == MOE_DTYPE_F32)
+    // dynamic shared memory: the value histogram of rows of bf16 values, or the buckets of the fp32 order
+    constexpr size_t histogram_bytes = sizeof(uint32_t) * kHistogramBins;
+    static_assert(histogram_bytes >= kOrderSharedBytes, "deferred fp32 rows use either");
+    // kept lists need the materialised order, rows with a large Top-K their own list length: neither is for clusters
+    if (args.dtype == MOE_DTYPE_F32 && untruncated_rows != 0 && args.kept_count == nullptr)
+    {
+        if (cudaError_t status = launch_sample_exact_cluster(args, ws, untruncated_rows, stream))
+            return status;
+        static SharedOptIn opt_in;
+        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<float, true>, histogram_bytes))
+            return status;
+        sample_exact_kernel<float, true><<<grid, kExactThreads, histogram_bytes, stream>>>(args, ws);
+    }
+    else if (args.dtype == MOE_DTYPE_F32)
     {
         static SharedOptIn opt_in;
-        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<float>, kOrderSharedBytes))
+        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<float, false>, kOrderSharedBytes))
             return status;
-        sample_exact_kernel<float><<<grid, kExactThreads, kOrderSharedBytes, stream>>>(args, ws);
+        sample_exact_kernel<float, false><<<grid, kExactThreads, kOrderSharedBytes, stream>>>(args, ws);
     }
     else
     {
-        // the value histogram of the bf16 path lives in dynamic shared memory
-        const size_t shared_bytes = sizeof(uint32_t) * kHistogramBins;
         static SharedOptIn opt_in;
-        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<__nv_bfloat16>, shared_bytes))
+        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<__nv_bfloat16, false>, histogram_bytes))
             return status;
-        sample_exact_kernel<__nv_bfloat16><<<grid, kExactThreads, shared_bytes, stream>>>(args, ws);
+        sample_exact_kernel<__nv_bfloat16, false><<<grid, kExactThreads, histogram_bytes, stream>>>(args, ws);
     }
     return cudaGetLastError();
 }
