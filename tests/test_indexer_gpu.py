@@ -54,3 +54,25 @@ def test_limits(sampler, pkg, torch_cuda):
     indices = sampler.indexer_topk(scores, 16)          # more than there are entries
     torch.cuda.synchronize()
     assert indices.cpu().numpy()[0].tolist() == list(range(10)) + [-1] * 6
+
+
+@pytest.mark.parametrize("count,top_k", [(1025, 1024), (2049, 2047), (5000, 2500), (10001, 5000), (40448, 512), (40449, 2048), (50001, 8192)])
+def test_boundaries_of_the_selection(sampler, checker, torch_cuda, count, top_k):
+    """Every way the k-th key can be found (few keys share its leading digit, only zeros do, many equal or nearly equal
+    ones do) and every way the selection is put in order (buckets, the network for piled-up keys), at the sizes where
+    the row stops fitting shared memory and the lists change their length; rows of every 16-byte phase."""
+    rng = np.random.default_rng(count)
+    rows = np.empty((9, count + 3), dtype=np.float32)                                   # odd stride: every phase
+    normal = rng.standard_normal((9, count + 3)).astype(np.float32)
+    rows[0] = normal[0]
+    rows[1] = np.maximum(normal[1], 0.0)                                                # half zeros
+    rows[2] = np.where(rng.random(count + 3) < 0.02, normal[2], 0.0)                    # the boundary lies among the zeros
+    rows[3] = np.where(normal[3] > 0.0, normal[3] * 1e-41, 0.0)                         # denormals share the zeros' digit
+    rows[4] = np.round(normal[4] * 2.0) / 2.0                                           # a few values
+    rows[5] = 1.0 + 1e-6 * normal[5]                                                    # nearly equal: the later digits decide
+    rows[6] = np.where(rng.random(count + 3) < 0.5, -0.0, -np.abs(normal[6]))           # zeros on top, negative rest
+    rows[7] = 7.25                                                                      # all equal
+    rows[8] = normal[8]
+    rows[8, rng.choice(count, 40, replace=False)] = np.inf
+    rows[8, rng.choice(count, 40, replace=False)] = -np.inf
+    check(sampler, checker, torch_cuda, rows, top_k, count=count)
