@@ -214,6 +214,14 @@ __device__ __forceinline__ const T* row_logits(const Args& a, uint32_t row)
     return static_cast<const T*>(a.logits) + static_cast<size_t>(row) * a.row_stride;
 }
 
+// ---- programmatic stream serialization -------------------------------------------
+// Waits until the kernel before this one in the stream has completed and its writes are visible; returns at once in a
+// kernel that was launched the ordinary way.
+__device__ __forceinline__ void wait_for_previous_kernel()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---- warp / block reductions ------------------------------------------------------
 __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v)
 {

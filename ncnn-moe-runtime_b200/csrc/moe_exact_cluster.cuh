@@ -1189,6 +1189,7 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
     const uint32_t rank = cluster.block_rank();
     const uint32_t cluster_size = cluster.num_blocks();
     const uint32_t tid = threadIdx.x;
+    wait_for_previous_kernel();
     const uint32_t pending = *ws.exact_count;
     const uint32_t slot_stride = (ws.max_vocab + 3u) & ~3u;
     // the cluster's items (numerators, then group numbers), every CTA its slice; padded so that slices stay 16-byte aligned
@@ -1277,7 +1278,7 @@ cudaError_t launch_sample_exact_cluster(const SampleArgs& args, const Workspace&
     config.blockDim = dim3(kExactThreads, 1, 1);
     config.dynamicSmemBytes = kClusterSharedBytes;
     config.stream = stream;
-    cudaLaunchAttribute attribute[1];
+    cudaLaunchAttribute attribute[2];
     attribute[0].id = cudaLaunchAttributeClusterDimension;
     attribute[0].val.clusterDim.y = 1;
     attribute[0].val.clusterDim.z = 1;
@@ -1332,6 +1333,8 @@ cudaError_t launch_sample_exact_cluster(const SampleArgs& args, const Workspace&
     const uint32_t clusters = rows < resident ? rows : resident;
     attribute[0].val.clusterDim.x = size;
     config.gridDim = dim3(clusters * size, 1, 1);
+    attribute[1] = follow_closely();
+    config.numAttrs = 2;
     return cudaLaunchKernelEx(&config, sample_exact_cluster_kernel, args, ws);
 }
 

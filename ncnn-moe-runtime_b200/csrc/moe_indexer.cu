@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(kIndexThreads) indexer_topk_kernel(const float
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
+    wait_for_previous_kernel();
     const float* row = scores + static_cast<size_t>(blockIdx.x) * row_stride;
     const uint32_t selected = min(top_k, count);
     out_index += static_cast<size_t>(blockIdx.x) * top_k;
@@ -570,8 +571,8 @@ cudaError_t launch_indexer(const float* scores, uint32_t rows, uint32_t count, s
     static SharedOptIn opt_in;
     if (cudaError_t status = opt_in_shared(opt_in, indexer_topk_kernel<kItems>, shared_bytes))
         return status;
-    indexer_topk_kernel<kItems><<<rows, kIndexThreads, shared_bytes, stream>>>(scores, count, row_stride, top_k, resident_fours, out_index, out_score);
-    return cudaGetLastError();
+    return launch_following(indexer_topk_kernel<kItems>, rows, kIndexThreads, shared_bytes, stream, scores, count, row_stride, top_k, resident_fours, out_index,
+                            out_score);
 }
 
 } // namespace

@@ -1414,6 +1414,7 @@ template<typename T, bool kDeferred>
 __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_kernel(const SampleArgs a, Workspace ws)
 {
     __shared__ ExactShared sh;
+    wait_for_previous_kernel();
     uint32_t* const count = kDeferred ? ws.exact_deferred_count : ws.exact_count;
     const uint32_t* const entries = kDeferred ? ws.exact_deferred : ws.exact_rows;
     const uint32_t pending = *count;
@@ -1446,41 +1447,32 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_kernel(const Sa
     }
 }
 
+template<typename T, bool kDeferred>
+cudaError_t launch_alone(const SampleArgs& args, const Workspace& ws, size_t shared_bytes, cudaStream_t stream)
+{
+    static SharedOptIn opt_in;
+    if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<T, kDeferred>, shared_bytes))
+        return status;
+    return launch_following(sample_exact_kernel<T, kDeferred>, ws.slots < args.rows ? ws.slots : args.rows, kExactThreads, shared_bytes, stream, args, ws);
+}
+
 } // namespace
 
 cudaError_t launch_sample_exact(const SampleArgs& args, const Workspace& ws, uint32_t untruncated_rows, cudaStream_t stream)
 {
     if (args.rows == 0 || ws.slots == 0)
         return cudaSuccess;
-    const uint32_t grid = ws.slots < args.rows ? ws.slots : args.rows;
     // dynamic shared memory: the value histogram of rows of bf16 values, or the buckets of the fp32 order
     constexpr size_t histogram_bytes = sizeof(uint32_t) * kHistogramBins;
     static_assert(histogram_bytes >= kOrderSharedBytes, "deferred fp32 rows use either");
+    if (args.dtype != MOE_DTYPE_F32)
+        return launch_alone<__nv_bfloat16, false>(args, ws, histogram_bytes, stream);
     // kept lists need the materialised order, rows with a large Top-K their own list length: neither is for clusters
-    if (args.dtype == MOE_DTYPE_F32 && untruncated_rows != 0 && args.kept_count == nullptr)
-    {
-        if (cudaError_t status = launch_sample_exact_cluster(args, ws, untruncated_rows, stream))
-            return status;
-        static SharedOptIn opt_in;
-        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<float, true>, histogram_bytes))
-            return status;
-        sample_exact_kernel<float, true><<<grid, kExactThreads, histogram_bytes, stream>>>(args, ws);
-    }
-    else if (args.dtype == MOE_DTYPE_F32)
-    {
-        static SharedOptIn opt_in;
-        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<float, false>, kOrderSharedBytes))
-            return status;
-        sample_exact_kernel<float, false><<<grid, kExactThreads, kOrderSharedBytes, stream>>>(args, ws);
-    }
-    else
-    {
-        static SharedOptIn opt_in;
-        if (cudaError_t status = opt_in_shared(opt_in, sample_exact_kernel<__nv_bfloat16, false>, histogram_bytes))
-            return status;
-        sample_exact_kernel<__nv_bfloat16, false><<<grid, kExactThreads, histogram_bytes, stream>>>(args, ws);
-    }
-    return cudaGetLastError();
+    if (untruncated_rows == 0 || args.kept_count != nullptr)
+        return launch_alone<float, false>(args, ws, kOrderSharedBytes, stream);
+    if (cudaError_t status = launch_sample_exact_cluster(args, ws, untruncated_rows, stream))
+        return status;
+    return launch_alone<float, true>(args, ws, histogram_bytes, stream);
 }
 
 } // namespace moe

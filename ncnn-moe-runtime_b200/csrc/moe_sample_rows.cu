@@ -113,10 +113,6 @@ namespace {
 // Programmatic dependent launch (sm_90+).  `wait` blocks until every kernel this
 // launch depends on has completed and its memory is visible; `launch_dependents`
 // lets the next kernel of the stream begin once all CTAs have issued it or exited.
-__device__ __forceinline__ void grid_dependency_wait()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 __device__ __forceinline__ void grid_dependency_release()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1475,6 +1471,8 @@ __global__ void __launch_bounds__(kThreads, MOE_ROW_MIN_CTAS) sample_rows_kernel
     // their own logits while this grid finishes.
     if (a.overlap_previous)
         grid_dependency_release();
+    else
+        wait_for_previous_kernel();
 
     // ---- the slice of this CTA, and its first bytes on request at once -----------
     const T* row_pointer = row_logits<T>(a, row);
@@ -1540,7 +1538,7 @@ __global__ void __launch_bounds__(kThreads, MOE_ROW_MIN_CTAS) sample_rows_kernel
         ring_drain(ring);
         // every CTA of the row takes this branch, so the arrival counter stays untouched
         if (a.overlap_previous)
-            grid_dependency_wait();
+            wait_for_previous_kernel();
         if (rank == 0)
         {
             if (tid == 0)
@@ -1614,7 +1612,7 @@ __global__ void __launch_bounds__(kThreads, MOE_ROW_MIN_CTAS) sample_rows_kernel
         // Everything up to here only read the logits and the row parameters.  The
         // slots, counters and outputs below may still be in use by the previous
         // launch: wait until it has completed.
-        grid_dependency_wait();
+        wait_for_previous_kernel();
     }
 
     if (splits > 1)
@@ -1715,6 +1713,7 @@ __global__ void __launch_bounds__(kThreads, 2) merge_candidates_kernel(const uin
     float* const scratch = reinterpret_cast<float*>(records + kCapLarge);
     const uint32_t row = blockIdx.x;
     const int tid = threadIdx.x;
+    wait_for_previous_kernel();
     const moe_row_params p = a.params[row];
     int invalid = validate_row(p);
     if (invalid == MOE_ROW_OK && p.temperature != 0.0f && p.top_k != top_k)
@@ -1795,22 +1794,7 @@ cudaError_t launch_typed(const SampleArgs& args, const Workspace& ws, uint32_t s
     cudaError_t status = opt_in_shared(opt_in, sample_rows_kernel<T, kLargeBuffer>, shared_bytes);
     if (status != cudaSuccess)
         return status;
-    if (!args.overlap_previous)
-    {
-        sample_rows_kernel<T, kLargeBuffer><<<args.rows * splits, kThreads, shared_bytes, stream>>>(args, ws, splits, stages);
-        return cudaGetLastError();
-    }
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(args.rows * splits, 1, 1);
-    config.blockDim = dim3(kThreads, 1, 1);
-    config.dynamicSmemBytes = shared_bytes;
-    config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attribute;
-    config.numAttrs = 1;
-    return cudaLaunchKernelEx(&config, sample_rows_kernel<T, kLargeBuffer>, args, ws, splits, stages);
+    return launch_following(sample_rows_kernel<T, kLargeBuffer>, args.rows * splits, kThreads, shared_bytes, stream, args, ws, splits, stages);
 }
 
 // Ring slots per warp and CTAs per SM that go with them.  Two CTAs per SM with
@@ -1874,8 +1858,7 @@ cudaError_t launch_merge_candidates(const uint64_t* gathered, uint32_t shards, u
     a.row_status = row_status;
     a.topk_index = topk_index;
     a.topk_stride = topk_stride;
-    merge_candidates_kernel<<<rows, kThreads, shared_bytes, stream>>>(gathered, shards, rows, top_k, a);
-    return cudaGetLastError();
+    return launch_following(merge_candidates_kernel, rows, kThreads, shared_bytes, stream, gathered, shards, rows, top_k, a);
 }
 
 uint32_t choose_splits(uint32_t rows, uint32_t vocab, int dtype, int sm_count, uint32_t slice_slots, bool large_top_k, bool overlapped)

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kVerifyThreads, 1) speculative_verify_kernel(c
     const int warp = tid >> 5;
     const uint32_t n = s.draft_count;
     const uint32_t session = blockIdx.x;
+    wait_for_previous_kernel();
     // rows of the sampler outputs: every Session's draft_count + 1 target positions first, then every Session's draft positions
     const uint32_t target_first = session * (n + 1u);
     const uint32_t draft_first = s.sessions * (n + 1u) + session * n;
@@ -344,8 +345,7 @@ __global__ void __launch_bounds__(kVerifyThreads, 1) speculative_verify_kernel(c
 
 cudaError_t launch_speculative_verify(const SpeculativeArgs& args, cudaStream_t stream)
 {
-    speculative_verify_kernel<<<args.sessions, kVerifyThreads, 0, stream>>>(args);
-    return cudaGetLastError();
+    return launch_following(speculative_verify_kernel, args.sessions, kVerifyThreads, 0, stream, args);
 }
 
 } // namespace moe
