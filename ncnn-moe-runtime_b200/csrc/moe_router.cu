@@ -23,6 +23,8 @@
 
 #include <cstdio>
 
+#include <cooperative_groups.h>
+
 #include "moe_common.cuh"
 #include "moe_internal.h"
 
@@ -152,126 +154,118 @@ __device__ __forceinline__ void warp_radix_select(uint64_t* records, uint32_t n,
     }
 }
 
-__global__ void __launch_bounds__(kRouteThreads) router_select_kernel(const RouterArgs a, unsigned long long* error_word)
+// Scores one token, selects its experts and their weights (out_expert, out_weight: top_k entries of this token) and
+// counts them in block_counts.  One warp; scores and records hold expert_count entries, radix_bins 256 (wide routers only).
+__device__ __forceinline__ void select_token(const RouterArgs& a, uint32_t token, float* scores, uint64_t* records, uint32_t* radix_bins,
+                                             uint32_t* block_counts, unsigned long long* error_word, uint32_t* out_expert, float* out_weight)
 {
-    extern __shared__ __align__(16) unsigned char shared_raw[];
     const uint32_t experts = a.options.expert_count;
     const uint32_t top_k = a.options.top_k;
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    // shared: scores [warps][experts] | records [warps][experts] | block counts [experts] | radix bins [warps][256]
-    float* scores = reinterpret_cast<float*>(shared_raw) + static_cast<size_t>(warp) * experts;
-    uint64_t* records = reinterpret_cast<uint64_t*>(shared_raw + sizeof(float) * experts * kRouteWarps) + static_cast<size_t>(warp) * experts;
-    uint32_t* block_counts = reinterpret_cast<uint32_t*>(shared_raw + (sizeof(float) + sizeof(uint64_t)) * experts * kRouteWarps);
-    uint32_t* radix_bins = block_counts + experts + warp * 256;
     const bool renormalize = (a.options.flags & MOE_ROUTER_FLAG_NORMALIZE_TOPK) != 0 || a.options.normalization == 1;
     const bool wide = experts > kNarrowExperts || top_k > kNarrowTopK;
-
-    for (uint32_t e = threadIdx.x; e < experts; e += kRouteThreads)
-        block_counts[e] = 0;
-    __syncthreads();
-
-    const uint32_t token_begin = blockIdx.x * a.tokens_per_block;
-    const uint32_t token_end = min(a.token_count, token_begin + a.tokens_per_block);
-    for (uint32_t token = token_begin + warp; token < token_end; token += kRouteWarps)
+    const float* logits = a.logits + static_cast<size_t>(token) * experts;
+    bool bad = false;
+    float peak = -INFINITY;
+    for (uint32_t e = lane; e < experts; e += 32)
     {
-        const float* logits = a.logits + static_cast<size_t>(token) * experts;
-        bool bad = false;
-        float peak = -INFINITY;
+        const float v = logits[e];
+        bad |= !(fabsf(v) < INFINITY);
+        peak = fmaxf(peak, v);
+    }
+    if (__any_sync(kFullMask, bad))
+    {
+        if (lane == 0)
+            report_error(error_word, 0, 0, 101);
+        return;
+    }
+    if (a.options.score_function == MOE_ROUTER_SOFTMAX)
+    {
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1)
+            peak = fmaxf(peak, __shfl_xor_sync(kFullMask, peak, offset));
+        float total = 0.0f;
+        for (uint32_t base = 0; base < experts; base += 32)
+        {
+            const uint32_t e = base + lane;
+            float weight = 0.0f;
+            if (e < experts)
+            {
+                weight = exact_expf(__fsub_rn(logits[e], peak));
+                scores[e] = weight;
+            }
+            // index order, :47-51; the padding adds zero.  Unrolled: the shuffles do not wait for the adds
+#pragma unroll
+            for (uint32_t j = 0; j < 32u; ++j)
+                total = __fadd_rn(total, __shfl_sync(kFullMask, weight, j));
+        }
+        __syncwarp();
+        for (uint32_t e = lane; e < experts; e += 32)
+            scores[e] = __fdiv_rn(scores[e], total);
+    }
+    else
+    {
         for (uint32_t e = lane; e < experts; e += 32)
         {
             const float v = logits[e];
-            bad |= !(fabsf(v) < INFINITY);
-            peak = fmaxf(peak, v);
+            float score;
+            if (a.options.score_function == MOE_ROUTER_SIGMOID)
+                score = __fdiv_rn(1.0f, __fadd_rn(1.0f, exact_expf(-v)));
+            else
+                score = __fsqrt_rn(router_softplus(v));
+            scores[e] = score;
         }
-        if (__any_sync(kFullMask, bad))
+    }
+    __syncwarp();
+
+    float chosen_total = 0.0f;
+    bool token_failed = false;
+    if (a.options.explicit_expert_ids != nullptr)
+    {
+        const uint32_t* explicit_ids = a.options.explicit_expert_ids + static_cast<size_t>(token) * top_k;
+        uint32_t first_bad = 0xFFFFFFFFu;
+        for (uint32_t r = lane; r < top_k; r += 32)
+        {
+            const uint32_t expert = explicit_ids[r];
+            if (expert >= experts)
+                first_bad = min(first_bad, r);
+            else
+                out_expert[r] = expert;
+        }
+        if (__any_sync(kFullMask, first_bad != 0xFFFFFFFFu))
         {
             if (lane == 0)
-                report_error(error_word, 0, 0, 101);
-            continue;
+                report_error(error_word, 1, token, 102);
+            token_failed = true;
         }
-        if (a.options.score_function == MOE_ROUTER_SOFTMAX)
+    }
+    else
+    {
+        bool nan_key = false;
+        for (uint32_t e = lane; e < experts; e += 32)
         {
-#pragma unroll
-            for (int offset = 16; offset > 0; offset >>= 1)
-                peak = fmaxf(peak, __shfl_xor_sync(kFullMask, peak, offset));
-            float total = 0.0f;
-            for (uint32_t base = 0; base < experts; base += 32)
-            {
-                const uint32_t e = base + lane;
-                float weight = 0.0f;
-                if (e < experts)
-                {
-                    weight = exact_expf(__fsub_rn(logits[e], peak));
-                    scores[e] = weight;
-                }
-                const uint32_t steps = min(32u, experts - base);
-                for (uint32_t j = 0; j < steps; ++j)
-                    total = __fadd_rn(total, __shfl_sync(kFullMask, weight, j)); // index order, :47-51
-            }
-            __syncwarp();
-            for (uint32_t e = lane; e < experts; e += 32)
-                scores[e] = __fdiv_rn(scores[e], total);
-        }
-        else
-        {
-            for (uint32_t e = lane; e < experts; e += 32)
-            {
-                const float v = logits[e];
-                float score;
-                if (a.options.score_function == MOE_ROUTER_SIGMOID)
-                    score = __fdiv_rn(1.0f, __fadd_rn(1.0f, exact_expf(-v)));
-                else
-                    score = __fsqrt_rn(router_softplus(v));
-                scores[e] = score;
-            }
+            const float key = (a.options.selection_bias != nullptr) ? __fadd_rn(scores[e], a.options.selection_bias[e]) : scores[e];
+            // NaN keys never win a `>` compare in the reference; rank them last
+            records[e] = (key == key) ? make_record(ordered_key(key), e) : 0ull;
+            nan_key |= !(key == key);
         }
         __syncwarp();
-
-        float chosen_total = 0.0f;
-        uint32_t* out_expert = a.selected_expert + static_cast<size_t>(token) * top_k;
-        float* out_weight = a.selected_weight + static_cast<size_t>(token) * top_k;
-        bool token_failed = false;
-        if (a.options.explicit_expert_ids != nullptr)
+        uint32_t pool = experts; // records the arg-max rounds look at
+        if (wide && top_k < experts && !__any_sync(kFullMask, nan_key))
         {
-            const uint32_t* explicit_ids = a.options.explicit_expert_ids + static_cast<size_t>(token) * top_k;
-            uint32_t first_bad = 0xFFFFFFFFu;
-            for (uint32_t r = lane; r < top_k; r += 32)
-            {
-                const uint32_t expert = explicit_ids[r];
-                if (expert >= experts)
-                    first_bad = min(first_bad, r);
-                else
-                    out_expert[r] = expert;
-            }
-            if (__any_sync(kFullMask, first_bad != 0xFFFFFFFFu))
-            {
-                if (lane == 0)
-                    report_error(error_word, 1, token, 102);
-                token_failed = true;
-            }
+            warp_radix_select(records, experts, top_k, radix_bins);
+            pool = top_k;
         }
-        else
+        // every lane keeps the best of its records; only the lane that owned a winner looks again
+        uint64_t best = 0ull;
+        uint32_t best_slot = 0;
+        bool look = true;
+        for (uint32_t r = 0; r < top_k; ++r)
         {
-            bool nan_key = false;
-            for (uint32_t e = lane; e < experts; e += 32)
+            if (look)
             {
-                const float key = (a.options.selection_bias != nullptr) ? __fadd_rn(scores[e], a.options.selection_bias[e]) : scores[e];
-                // NaN keys never win a `>` compare in the reference; rank them last
-                records[e] = (key == key) ? make_record(ordered_key(key), e) : 0ull;
-                nan_key |= !(key == key);
-            }
-            __syncwarp();
-            uint32_t pool = experts; // records the arg-max rounds look at
-            if (wide && top_k < experts && !__any_sync(kFullMask, nan_key))
-            {
-                warp_radix_select(records, experts, top_k, radix_bins);
-                pool = top_k;
-            }
-            for (uint32_t r = 0; r < top_k; ++r)
-            {
-                uint64_t best = 0ull;
-                uint32_t best_slot = 0;
+                best = 0ull;
+#pragma unroll 4
                 for (uint32_t i = lane; i < pool; i += 32)
                 {
                     const uint64_t record = records[i];
@@ -281,49 +275,74 @@ __global__ void __launch_bounds__(kRouteThreads) router_select_kernel(const Rout
                         best_slot = i;
                     }
                 }
-                const uint32_t best_hi = __reduce_max_sync(kFullMask, static_cast<uint32_t>(best >> 32));
-                const uint32_t candidate_lo = (static_cast<uint32_t>(best >> 32) == best_hi) ? static_cast<uint32_t>(best) : 0u;
-                const uint32_t best_lo = __reduce_max_sync(kFullMask, candidate_lo);
-                const bool mine = best != 0ull && static_cast<uint32_t>(best >> 32) == best_hi && static_cast<uint32_t>(best) == best_lo;
-                uint32_t expert = 0xFFFFFFFFu - best_lo;
-                if (expert >= experts)
-                    expert = 0; // only when every remaining key is NaN
-                if (mine)
-                    records[best_slot] = 0ull; // records are unique: exactly one lane owns the winner
-                if (lane == 0)
-                    out_expert[r] = expert;
-                __syncwarp();
             }
-        }
-        if (token_failed)
-            continue;
-        __syncwarp();
-        __threadfence_block();
-        // rank-order sequential sum of the unbiased scores (:131-133)
-        for (uint32_t base = 0; base < top_k; base += 32)
-        {
-            const uint32_t r = base + lane;
-            const float score = (r < top_k) ? scores[out_expert[r]] : 0.0f;
-            const uint32_t steps = min(32u, top_k - base);
-            for (uint32_t j = 0; j < steps; ++j)
-                chosen_total = __fadd_rn(chosen_total, __shfl_sync(kFullMask, score, j));
-        }
-        if (renormalize && chosen_total <= 0.0f)
-        {
+            const uint32_t best_hi = __reduce_max_sync(kFullMask, static_cast<uint32_t>(best >> 32));
+            const uint32_t candidate_lo = (static_cast<uint32_t>(best >> 32) == best_hi) ? static_cast<uint32_t>(best) : 0u;
+            const uint32_t best_lo = __reduce_max_sync(kFullMask, candidate_lo);
+            const bool mine = best != 0ull && static_cast<uint32_t>(best >> 32) == best_hi && static_cast<uint32_t>(best) == best_lo;
+            uint32_t expert = 0xFFFFFFFFu - best_lo;
+            if (expert >= experts)
+                expert = 0; // only when every remaining key is NaN
+            if (mine)
+                records[best_slot] = 0ull; // records are unique: exactly one lane owns the winner
+            look = mine;
             if (lane == 0)
-                report_error(error_word, 1, token, 103);
-            continue;
+                out_expert[r] = expert;
+            __syncwarp();
         }
-        for (uint32_t r = lane; r < top_k; r += 32)
-        {
-            const uint32_t expert = out_expert[r];
-            const float score = scores[expert];
-            const float weight = __fmul_rn(renormalize ? __fdiv_rn(score, chosen_total) : score, a.options.routed_scaling_factor);
-            out_weight[r] = weight;
-            atomicAdd(&block_counts[expert], 1u);
-        }
-        __syncwarp();
     }
+    if (token_failed)
+        return;
+    __syncwarp();
+    __threadfence_block();
+    // rank-order sequential sum of the unbiased scores (:131-133)
+    for (uint32_t base = 0; base < top_k; base += 32)
+    {
+        const uint32_t r = base + lane;
+        const float score = (r < top_k) ? scores[out_expert[r]] : 0.0f;
+        const uint32_t steps = min(32u, top_k - base);
+#pragma unroll 8
+        for (uint32_t j = 0; j < steps; ++j)
+            chosen_total = __fadd_rn(chosen_total, __shfl_sync(kFullMask, score, j));
+    }
+    if (renormalize && chosen_total <= 0.0f)
+    {
+        if (lane == 0)
+            report_error(error_word, 1, token, 103);
+        return;
+    }
+    for (uint32_t r = lane; r < top_k; r += 32)
+    {
+        const uint32_t expert = out_expert[r];
+        const float score = scores[expert];
+        const float weight = __fmul_rn(renormalize ? __fdiv_rn(score, chosen_total) : score, a.options.routed_scaling_factor);
+        out_weight[r] = weight;
+        atomicAdd(&block_counts[expert], 1u);
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(kRouteThreads) router_select_kernel(const RouterArgs a, unsigned long long* error_word)
+{
+    extern __shared__ __align__(16) unsigned char shared_raw[];
+    const uint32_t experts = a.options.expert_count;
+    const uint32_t top_k = a.options.top_k;
+    const int warp = threadIdx.x >> 5;
+    // shared: scores [warps][experts] | records [warps][experts] | block counts [experts] | radix bins [warps][256]
+    float* scores = reinterpret_cast<float*>(shared_raw) + static_cast<size_t>(warp) * experts;
+    uint64_t* records = reinterpret_cast<uint64_t*>(shared_raw + sizeof(float) * experts * kRouteWarps) + static_cast<size_t>(warp) * experts;
+    uint32_t* block_counts = reinterpret_cast<uint32_t*>(shared_raw + (sizeof(float) + sizeof(uint64_t)) * experts * kRouteWarps);
+    uint32_t* radix_bins = block_counts + experts + warp * 256;
+
+    for (uint32_t e = threadIdx.x; e < experts; e += kRouteThreads)
+        block_counts[e] = 0;
+    __syncthreads();
+
+    const uint32_t token_begin = blockIdx.x * a.tokens_per_block;
+    const uint32_t token_end = min(a.token_count, token_begin + a.tokens_per_block);
+    for (uint32_t token = token_begin + warp; token < token_end; token += kRouteWarps)
+        select_token(a, token, scores, records, radix_bins, block_counts, error_word, a.selected_expert + static_cast<size_t>(token) * top_k,
+                     a.selected_weight + static_cast<size_t>(token) * top_k);
     __syncthreads();
     // this block's column of the [expert][block] table
     for (uint32_t e = threadIdx.x; e < experts; e += kRouteThreads)
@@ -452,48 +471,188 @@ __global__ void __launch_bounds__(kRouteThreads) router_place_kernel(const Route
     }
 }
 
-__global__ void __launch_bounds__(256) regroup_gather_kernel(const float* hidden, uint32_t token_count, uint32_t columns, const uint32_t* route_token,
-                                                             uint32_t route_count, float* gathered, int32_t* out_of_range, int vectorised)
+// The whole dispatch of a few tokens in one launch: a cluster of kFewCtas CTAs, one warp per token.  Each CTA owns
+// a contiguous run of tokens and keeps its routes and their counts in shared memory; after one cluster barrier it
+// reads its peers' counts, scans the totals into CSR offsets and places its own routes.
+// What bounds it: the latency of one token's selection (exp, k arg-max rounds) and of the launch; three launches with
+// a table in global memory between them cost 11.7 us for 32 tokens of 128 experts (7.7 here), 17.4 for 64 of 256 (11.6).
+constexpr uint32_t kFewCtas = 8;
+constexpr uint32_t kFewThreads = 512;
+constexpr uint32_t kFewWarps = kFewThreads / 32;
+constexpr uint32_t kFewTokens = kFewCtas * kFewWarps; // one round: with two the three launches over all SMs win (192 tokens: 24.9 against 18.1 us)
+constexpr uint32_t kFewTokensPerCta = kFewTokens / kFewCtas;
+
+size_t few_shared_bytes(uint32_t experts, uint32_t top_k)
 {
-    // one warp per route row keeps each copy a run of full 128-byte lines
-    const uint32_t warps_per_block = 256 / 32;
+    return (sizeof(float) + sizeof(uint64_t)) * experts * kFewWarps + 2u * sizeof(uint32_t) * experts + 2u * sizeof(uint32_t) * kFewTokensPerCta * top_k;
+}
+
+__global__ void __cluster_dims__(kFewCtas, 1, 1) __launch_bounds__(kFewThreads) router_few_tokens_kernel(const RouterArgs a)
+{
+    extern __shared__ __align__(16) unsigned char shared_raw[];
+    __shared__ unsigned long long error_word;
+    __shared__ uint32_t warp_total[kFewWarps];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t experts = a.options.expert_count;
+    const uint32_t top_k = a.options.top_k;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t lane = tid & 31u;
+    const uint32_t warp = tid >> 5;
+    const uint32_t rank = cluster.block_rank();
+    // records [warps][experts] | scores [warps][experts] | counts [experts] | base [experts] | route experts | route weights
+    uint64_t* records = reinterpret_cast<uint64_t*>(shared_raw) + static_cast<size_t>(warp) * experts;
+    float* all_scores = reinterpret_cast<float*>(shared_raw + sizeof(uint64_t) * experts * kFewWarps);
+    float* scores = all_scores + static_cast<size_t>(warp) * experts;
+    uint32_t* counts = reinterpret_cast<uint32_t*>(all_scores + static_cast<size_t>(kFewWarps) * experts);
+    uint32_t* base = counts + experts;
+    uint32_t* route_expert = base + experts;
+    float* route_weight = reinterpret_cast<float*>(route_expert + kFewTokensPerCta * top_k);
+
+    for (uint32_t e = tid; e < experts; e += kFewThreads)
+        counts[e] = 0;
+    if (tid == 0)
+        error_word = ~0ull;
+    wait_for_previous_kernel();
+    __syncthreads();
+    const uint32_t per = (a.token_count + kFewCtas - 1u) / kFewCtas;
+    const uint32_t token_begin = min(a.token_count, rank * per);
+    const uint32_t token_end = min(a.token_count, token_begin + per);
+    for (uint32_t token = token_begin + warp; token < token_end; token += kFewWarps)
+        select_token(a, token, scores, records, nullptr, counts, &error_word, route_expert + (token - token_begin) * top_k,
+                     route_weight + (token - token_begin) * top_k);
+    cluster.sync();
+
+    unsigned long long error = ~0ull;
+    for (uint32_t r = 0; r < kFewCtas; ++r)
+        error = min(error, *cluster.map_shared_rank(&error_word, r));
+    uint32_t carry = 0;
+    for (uint32_t first = 0; first < experts; first += kFewThreads)
+    {
+        const uint32_t e = first + tid;
+        uint32_t total = 0, before = 0;
+        if (e < experts)
+        {
+#pragma unroll
+            for (uint32_t r = 0; r < kFewCtas; ++r)
+            {
+                const uint32_t n = cluster.map_shared_rank(counts, r)[e];
+                total += n;
+                before += r < rank ? n : 0u;
+            }
+        }
+        uint32_t scan = total;
+#pragma unroll
+        for (int offset = 1; offset < 32; offset <<= 1)
+        {
+            const uint32_t other = __shfl_up_sync(kFullMask, scan, offset);
+            if (lane >= static_cast<uint32_t>(offset))
+                scan += other;
+        }
+        if (lane == 31)
+            warp_total[warp] = scan;
+        __syncthreads();
+        const uint32_t of_warp = lane < kFewWarps ? warp_total[lane] : 0u;
+        const uint32_t offset = carry + __reduce_add_sync(kFullMask, lane < warp ? of_warp : 0u) + scan - total;
+        carry += __reduce_add_sync(kFullMask, of_warp);
+        if (e < experts)
+        {
+            base[e] = offset + before;
+            if (rank == 0)
+                a.expert_offsets[e] = offset;
+        }
+        __syncthreads();
+    }
+    if (rank == 0 && tid == 0)
+    {
+        a.expert_offsets[experts] = carry;
+        a.plan_status[0] = error == ~0ull ? 0 : static_cast<int32_t>(error & 0xFFu);
+    }
+    cluster.sync(); // the peers have read this CTA's counts
+    if (error != ~0ull)
+        return; // a failed call leaves no plan
+    const uint32_t routes = (token_end - token_begin) * top_k;
+    for (uint32_t i = tid; i < routes; i += kFewThreads)
+    {
+        const uint32_t expert = route_expert[i];
+        uint32_t earlier = 0; // routes of this expert before mine, in (token, rank) order
+#pragma unroll 4
+        for (uint32_t j = 0; j < i; ++j)
+            earlier += route_expert[j] == expert ? 1u : 0u;
+        const uint32_t slot = base[expert] + earlier;
+        a.route_token[slot] = token_begin + i / top_k;
+        a.route_rank[slot] = i % top_k;
+        a.route_weight[slot] = route_weight[i];
+    }
+}
+
+// One warp per piece of a route's row: 4 KiB (eight 16-byte loads in flight per lane, whole 128-byte lines), so that
+// a decode step's few rows spread over the SMs too; whole rows in calls that write more than L2 holds.
+// What bounds it: HBM writes; the hidden rows are read once per route of their token and stay in L2.  32768 rows of
+// 16 KiB: 126 us, 4.8 TB/s (bulk copies through shared memory: 135 us, and 39 against 24 us for rows of 4 KiB).
+// 128 rows of 11.25 KiB: 6.7 -> 5.4 us with pieces.
+constexpr uint32_t kGatherPiece = 8u * 32u; // 16-byte vectors
+
+__global__ void __launch_bounds__(256) regroup_gather_kernel(const float* hidden, uint32_t token_count, uint32_t columns, const uint32_t* route_token,
+                                                             uint32_t route_count, float* gathered, int32_t* out_of_range, int vectorised, uint32_t piece)
+{
+    wait_for_previous_kernel();
+    const uint32_t warps_per_block = blockDim.x / 32;
     const int lane = threadIdx.x & 31;
-    for (uint32_t route = blockIdx.x * warps_per_block + (threadIdx.x >> 5); route < route_count; route += gridDim.x * warps_per_block)
+    const uint32_t first = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
+    if (vectorised)
+    {
+        const uint32_t vectors = columns / 4;
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        // vectors [c, end) of a route's row, by the lanes of a warp; the copies leave with a streaming store so that the
+        // hidden rows stay in L2
+        const auto copy = [&](uint32_t route, uint32_t c, uint32_t end) {
+            const uint32_t token = route_token[route];
+            // a token index beyond the hidden matrix is never dereferenced: its row is zero-filled and the call flagged
+            const bool valid = token < token_count;
+            if (!valid && lane == 0)
+                *out_of_range = 1;
+            const float4* source = reinterpret_cast<const float4*>(hidden + static_cast<size_t>(valid ? token : 0u) * columns);
+            float4* target = reinterpret_cast<float4*>(gathered + static_cast<size_t>(route) * columns);
+            for (; c + 7u * 32u < end; c += 8u * 32u)
+            {
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    v[u] = valid ? __ldg(source + c + 32u * u) : zero;
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    __stcs(target + c + 32u * u, v[u]);
+            }
+            for (; c < end; c += 32)
+                __stcs(target + c, valid ? __ldg(source + c) : zero);
+        };
+        if (piece >= vectors)
+        {
+            for (uint32_t route = first; route < route_count; route += gridDim.x * warps_per_block)
+                copy(route, lane, vectors);
+            return;
+        }
+        const uint32_t pieces = (vectors + piece - 1u) / piece; // of a row
+        const uint64_t total = static_cast<uint64_t>(route_count) * pieces;
+        for (uint64_t item = first; item < total; item += gridDim.x * warps_per_block)
+        {
+            const uint32_t route = static_cast<uint32_t>(item / pieces);
+            const uint32_t begin = static_cast<uint32_t>(item - static_cast<uint64_t>(route) * pieces) * piece;
+            copy(route, begin + lane, min(vectors, begin + piece));
+        }
+        return;
+    }
+    for (uint32_t route = first; route < route_count; route += gridDim.x * warps_per_block)
     {
         const uint32_t token = route_token[route];
-        // a token index beyond the hidden matrix is never dereferenced: its row is zero-filled and the call flagged
         const bool valid = token < token_count;
         if (!valid && lane == 0)
             *out_of_range = 1;
         const float* source = hidden + static_cast<size_t>(valid ? token : 0u) * columns;
         float* target = gathered + static_cast<size_t>(route) * columns;
-        if (vectorised)
-        {
-            const float4* source4 = reinterpret_cast<const float4*>(source);
-            float4* target4 = reinterpret_cast<float4*>(target);
-            // eight 16-byte loads in flight per lane; the copies leave with a streaming store so that the
-            // hidden rows (read once per route of their token) stay in L2
-            const uint32_t vectors = columns / 4;
-            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            uint32_t c = lane;
-            for (; c + 7u * 32u < vectors; c += 8u * 32u)
-            {
-                float4 v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    v[u] = valid ? __ldg(source4 + c + 32u * u) : zero;
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    __stcs(target4 + c + 32u * u, v[u]);
-            }
-            for (; c < vectors; c += 32)
-                __stcs(target4 + c, valid ? __ldg(source4 + c) : zero);
-        }
-        else
-        {
-            for (uint32_t c = lane; c < columns; c += 32)
-                target[c] = valid ? source[c] : 0.0f;
-        }
+        for (uint32_t c = lane; c < columns; c += 32)
+            target[c] = valid ? source[c] : 0.0f;
     }
 }
 
@@ -504,6 +663,14 @@ cudaError_t launch_router_dispatch_kernels(const RouterArgs& caller_args, uint32
 {
     RouterArgs args = caller_args;
     const uint32_t experts = args.options.expert_count;
+    if (args.token_count <= kFewTokens && experts <= kNarrowExperts && args.options.top_k <= kNarrowTopK)
+    {
+        const size_t few_bytes = few_shared_bytes(experts, args.options.top_k);
+        static SharedOptIn few_opt_in;
+        if (cudaError_t status = opt_in_shared(few_opt_in, router_few_tokens_kernel, few_bytes))
+            return status;
+        return launch_following(router_few_tokens_kernel, kFewCtas, kFewThreads, few_bytes, stream, args);
+    }
     static_assert(kRouteWarps == 4, "router_partition_host assumes four warps per block");
     const RouterPartition part = router_partition_host(args.token_count, experts);
     args.tokens_per_block = part.tokens_per_block;
@@ -528,10 +695,17 @@ cudaError_t launch_regroup_gather(const float* hidden, uint32_t token_count, uin
     if (route_count == 0 || columns == 0)
         return cudaSuccess;
     const int vectorised = (columns % 4 == 0) && ((reinterpret_cast<uintptr_t>(hidden) | reinterpret_cast<uintptr_t>(gathered)) % 16 == 0);
-    const uint32_t blocks_needed = (route_count + 7) / 8;
-    const uint32_t grid = blocks_needed < 148u * 16u ? blocks_needed : 148u * 16u;
-    regroup_gather_kernel<<<grid, 256, 0, stream>>>(hidden, token_count, columns, route_token, route_count, gathered, out_of_range, vectorised);
-    return cudaGetLastError();
+    // whole rows per warp once the copies outgrow L2 (32768 rows of 16 KiB: 126 against 134 us)
+    const bool whole_rows = static_cast<uint64_t>(route_count) * columns * sizeof(float) > (96ull << 20);
+    const uint32_t piece = whole_rows ? (columns + 3u) / 4u : kGatherPiece;
+    const uint64_t pieces = vectorised ? (columns / 4u + piece - 1u) / piece : 1u;
+    const uint64_t warps = static_cast<uint64_t>(route_count) * pieces;
+    // small calls: blocks of two warps, so that every SM gets some
+    const uint32_t threads = warps >= 148u * 16u ? 256u : 64u;
+    const uint64_t blocks_needed = (warps + threads / 32u - 1u) / (threads / 32u);
+    const uint32_t grid = blocks_needed < 148u * 16u ? static_cast<uint32_t>(blocks_needed) : 148u * 16u;
+    return launch_following(regroup_gather_kernel, grid, threads, 0, stream, hidden, token_count, columns, route_token, route_count, gathered, out_of_range,
+                            vectorised, piece);
 }
 
 

@@ -189,3 +189,39 @@ def test_router_errors(sampler, pkg):
     assert plan.status == 103 and pkg.library().moe_router_status_error_code(103) == 3
     # after a failed call the handle still works
     assert sampler.router_dispatch_host(logits, 4, 8, 2).status == 0
+
+
+@pytest.mark.parametrize("columns,routes", [(4, 444 * 33 + 5), (4, 445), (36, 444 * 32), (1024, 444 * 34 + 1), (4100, 1000), (8, 1), (6, 100)])
+def test_gather_moves_rows_in_pieces(sampler, torch_cuda, columns, routes):
+    """Row lengths from one 16-byte vector to several pieces, and as many pieces per warp as make its groups of ids and its
+    slots wrap; ids outside the matrix (their rows become zero, the call is flagged) between the others."""
+    torch = torch_cuda
+    generator = torch.Generator(device="cuda").manual_seed(columns + routes)
+    tokens = 97
+    hidden = torch.randn((tokens, columns), generator=generator, device="cuda")
+    ids = torch.randint(tokens, (routes,), generator=generator, device="cuda", dtype=torch.int32)
+    sampler.regroup_gather_check()
+    assert torch.equal(sampler.regroup_gather(hidden, ids), hidden[ids.long()])
+    assert not sampler.regroup_gather_check()
+    outside = torch.rand(routes, generator=generator, device="cuda") < 0.3
+    outside[-1] = True
+    broken = torch.where(outside, torch.full_like(ids, tokens), ids)
+    want = torch.where(outside[:, None], torch.zeros((), device="cuda"), hidden[ids.long()])
+    assert torch.equal(sampler.regroup_gather(hidden, broken), want)
+    assert sampler.regroup_gather_check()
+
+
+@pytest.mark.parametrize("tokens", [1, 7, 9, 128, 129, 255, 256, 257])
+@pytest.mark.parametrize("experts,top_k", [(3, 2), (511, 16), (513, 7), (1024, 8), (1025, 2)])
+def test_dispatch_around_the_one_launch_limits(sampler, checker, port, tokens, experts, top_k):
+    rng = np.random.default_rng(tokens * experts)
+    logits = (np.round(rng.standard_normal((tokens, experts)) * 8) / 8).astype(np.float32)          # many exact ties
+    bias = (0.1 * rng.standard_normal(experts)).astype(np.float32)
+    want, exact = both_oracles(checker, port, logits, tokens, experts, top_k, score_function=tokens % 3, selection_bias=bias)
+    plan = sampler.router_dispatch_host(logits, tokens, experts, top_k, score_function=tokens % 3, selection_bias=bias)
+    compare(plan, want, experts, exact["weight"])
+    if tokens > 1:
+        broken = logits.copy()
+        broken[tokens - 1, experts - 1] = np.nan
+        assert sampler.router_dispatch_host(broken, tokens, experts, top_k).status == 101           # non-finite logits
+        compare(sampler.router_dispatch_host(logits, tokens, experts, top_k, score_function=tokens % 3, selection_bias=bias), want, experts, exact["weight"])
