@@ -499,7 +499,7 @@ def run_speculative_bench(args, as_dict=False):
                              "sample": f"{len(cases)} verifications, single thread (a Session verifies on its own thread)"},
             "results_equal_to_reference": f"{equal}/{len(cases)}",
             "batched": {"sessions_per_call": sessions, "ms_per_call": batch_ms, "verifications_per_s": sessions * 1e3 / batch_ms,
-                        "logits_GBps": batch_bytes / batch_ms / 1e6, "kernels_per_call": 3, "steps": batch_steps,
+                        "logits_GBps": batch_bytes / batch_ms / 1e6, "kernels_per_call": 2, "steps": batch_steps,
                         "results_equal_to_reference": f"{batch_equal}/{sessions}"}}
     sampler.close()
     if as_dict:

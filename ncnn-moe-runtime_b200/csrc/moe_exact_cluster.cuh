@@ -649,6 +649,10 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                 ++finite;
                 low_bits |= __float_as_uint(v);
             }
+            else if (v != v && (__float_as_uint(v) & 0x007F0000u) == 0u)
+            {
+                low_bits |= 1u; // a NaN whose upper half alone would be an infinity
+            }
         };
         for_each_four(row_pointer, begin, end, [&](uint32_t, const float4& v) {
             see(v.x);

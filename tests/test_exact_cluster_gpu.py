@@ -40,3 +40,45 @@ def test_rows_finished_by_clusters(pkg, parity, copies, vocab):
     for step in range(3):
         params["step"] = step
         parity.check(logits, params)
+
+
+@pytest.mark.parametrize("stored", ["bf16", "widened"])
+@pytest.mark.parametrize("vocab", [33000, 129280])
+def test_rows_of_bf16_values_in_either_type(pkg, workloads, parity, stored, vocab):
+    """Rows of bf16 values, stored as bf16 or widened to fp32 (the clusters leave those to the value-run path): both give
+    the oracle's result, whatever the number of distinct values and the place where a sum ends."""
+    rng = np.random.default_rng(vocab)
+    rows = 40
+    values = rng.standard_normal((rows, vocab)).astype(np.float32) * rng.choice(np.array([0.3, 1.0, 2.0, 3.0, 5.0], dtype=np.float32), (rows, 1))
+    values[:10] += 8.0 * (rng.random((10, vocab)) < 0.0005)
+    values[10:14] = np.round(values[10:14] * 4.0) / 4.0
+    values[14:16] += 300.0
+    bits = workloads.to_bf16_bits(values)
+    logits = bits if stored == "bf16" else (bits.astype(np.uint32) << 16).view(np.float32)
+    params = pkg.make_row_params(rows, seed=vocab, top_k=0, temperature=rng.choice(np.array([0.7, 1.0, 1.3, 2.0], dtype=np.float32), rows),
+                                 top_p=rng.choice(np.array([0.6, 0.95, 1.0, 1.0], dtype=np.float32), rows),
+                                 min_p=rng.choice(np.array([0.0, 0.0, 1e-4], dtype=np.float32), rows))
+    for step in range(4):
+        params["step"] = step
+        parity.check(logits, params)
+
+
+def test_infinities_and_nans(pkg, parity):
+    """NaNs of any payload are skipped (one whose payload lies in the low half must not become an infinity in a row of
+    bf16 values), -inf is never chosen, +inf anywhere is the reference's error; a peak that overflows in the division by
+    the temperature gives an invalid distribution."""
+    rng = np.random.default_rng(5)
+    vocab = 40007
+    plain = (3.0 * rng.standard_normal(vocab)).astype(np.float32)
+    widened = ((plain.view(np.uint32) >> 16) << 16).view(np.float32)
+    rows = []
+    for base in (plain, widened):
+        quiet = base.copy(); quiet[rng.choice(vocab, 300, replace=False)] = np.nan; rows.append(quiet)
+        signalling = base.copy(); signalling.view(np.uint32)[rng.choice(vocab, 300, replace=False)] = 0x7F800001; rows.append(signalling)
+        masked = base.copy(); masked[rng.random(vocab) < 0.3] = -np.inf; rows.append(masked)
+        infinite = base.copy(); infinite[vocab - 1] = np.inf; rows.append(infinite)
+        huge = base.copy(); huge[:] = np.float32(3.0e38) - np.abs(base) * np.float32(1.0e32); rows.append(huge)
+    logits = np.stack(rows)
+    for temperature in (1.0, 0.5):
+        params = pkg.make_row_params(len(rows), seed=9, top_k=0, temperature=temperature, top_p=0.97)
+        parity.check(logits, params)
