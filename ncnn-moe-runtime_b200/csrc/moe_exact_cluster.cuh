@@ -126,6 +126,7 @@ struct alignas(16) ClusterShared
     LiteralGroup literal_in[kLiteralGroups];
     LiteralGroup literal[kLiteralGroups];
     uint32_t head_count, item_count, literal_count;
+    uint32_t literal_items; // items of the literal groups
     // every CTA
     ClusterStats stats[kMaxCluster];
     uint64_t cta_total[kMaxCluster];
@@ -831,6 +832,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
             {
                 cs.item_count = 0;
                 cs.literal_count = 0;
+                cs.literal_items = 0;
             }
             __syncthreads();
             const bool gather_head = sum == 0 && guess == 0;
@@ -927,13 +929,15 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                 }
                 if (literal)
                 {
-                    const uint32_t slot = atomicAdd(cluster.map_shared_rank(&cs.literal_count, 0), 1u);
+                    const uint32_t slot = atomicAdd(&first_cta.literal_count, 1u);
+                    atomicAdd(&first_cta.literal_items, static_cast<uint32_t>(cs.count[g]));
                     if (slot < kLiteralGroups)
                         cluster.map_shared_rank(cs.literal_in, 0)[slot] = LiteralGroup{before, running + correction, g, 0u};
                 }
             }
             cluster.sync();
-            const uint32_t literal_groups = *cluster.map_shared_rank(&cs.literal_count, 0);
+            const uint32_t literal_groups = first_cta.literal_count;
+            const uint32_t literal_items = first_cta.literal_items;
             CL_MARK(22);
             CL_COUNT(28, literal_groups);
             CL_COUNT(29, 1);
@@ -954,7 +958,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                         cluster.map_shared_rank(cs.exponent, r)[g] = exponent;
                 }
             };
-            if (literal_groups > kLiteralGroups)
+            if (literal_groups > kLiteralGroups || literal_items > kLiteralItems)
             {
                 // the guess was too far off: repeat with the exponents of the accumulators just found
                 publish_exponents(0u);
