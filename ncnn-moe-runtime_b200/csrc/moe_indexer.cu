@@ -16,9 +16,11 @@
 // inside each bucket, or, where keys pile up, by a bitonic network that runs in
 // registers for strides inside a warp and through shared memory for the others.
 //
-// What bounds it: latency and shared-memory instructions of one SM.  64 rows x
-// 40000 scores, top 2048: 82.0 us with byte digits, match.any aggregation, six
-// passes over L2 and a bitonic sort in shared memory; 28.7 us as it is here (128 rows x 131072: 263 -> 72; 64 rows x 2300: 30 -> 12).
+// What bounds it: latency and shared-memory instructions of one SM per row.  With
+// byte digits, match.any aggregation, six passes over L2 and a bitonic sort in
+// shared memory, before and after: 64 rows x 40000 scores, top 2048 82.0 -> 27.3 us;
+// 128 x 131072, top 2048 263 -> 72; 64 x 2300, top 2048 30 -> 12; 128 x 1024, top 512
+// 14 -> 11.
 
 #include "moe_common.cuh"
 #include "moe_internal.h"
