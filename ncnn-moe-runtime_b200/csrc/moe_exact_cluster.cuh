@@ -1268,15 +1268,10 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
 // rounds x (fixed + passes / size) wins.  Measured with clusters of 1, 2, 4, 8, 16 CTAs, us per call:
 // 1 row 253, 175, 137, 118, 112; 20 rows 355, 243, 190, 232, 324; 64 rows 420, 315, 378, 507, 855;
 // 256 rows 707, 750, 1032, 1680, 3193.
-struct ClusterOccupancy
-{
-    int active[5] = {0, 0, 0, 0, 0}; // resident clusters of 1, 2, 4, 8, 16 CTAs; 0: not asked yet
-};
-
 cudaError_t launch_sample_exact_cluster(const SampleArgs& args, const Workspace& ws, uint32_t untruncated_rows, cudaStream_t stream)
 {
     static SharedOptIn opt_in;
-    static ClusterOccupancy occupancy[kMaxDevices];
+    static ClusterOccupancyTable occupancy;
     if (cudaError_t status = opt_in_shared(opt_in, sample_exact_cluster_kernel, kClusterSharedBytes))
         return status;
     int device = 0;
@@ -1292,33 +1287,24 @@ cudaError_t launch_sample_exact_cluster(const SampleArgs& args, const Workspace&
     attribute[0].val.clusterDim.z = 1;
     config.attrs = attribute;
     config.numAttrs = 1;
-    ClusterOccupancy unknown;
-    ClusterOccupancy& known = device >= 0 && device < kMaxDevices ? occupancy[device] : unknown;
-    if (known.active[0] == 0)
-    {
-        if (cudaError_t status = cudaFuncSetAttribute(sample_exact_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
-            return status;
-        ClusterOccupancy found;
-        for (int i = 4; i >= 0; --i)
+    const ClusterOccupancy known = cluster_occupancy(occupancy, device, [&](int size_index, int* clusters) {
+        cudaError_t status = cudaFuncSetAttribute(sample_exact_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (status == cudaSuccess)
         {
-            attribute[0].val.clusterDim.x = 1u << i;
-            config.gridDim = dim3(1u << i, 1, 1);
-            if (cudaOccupancyMaxActiveClusters(&found.active[i], sample_exact_cluster_kernel, &config) != cudaSuccess)
-            {
-                (void)cudaGetLastError(); // this size is not available
-                found.active[i] = 0;
-            }
+            attribute[0].val.clusterDim.x = 1u << size_index;
+            config.gridDim = dim3(1u << size_index, 1, 1);
+            status = cudaOccupancyMaxActiveClusters(clusters, sample_exact_cluster_kernel, &config);
         }
-        if (found.active[0] < 1)
-            found.active[0] = 1;
-        known = found; // racing host threads write the same values
-    }
+        if (status != cudaSuccess)
+            (void)cudaGetLastError(); // this size is not available
+        return status;
+    });
     const uint32_t rows = untruncated_rows < args.rows ? untruncated_rows : args.rows;
     const double passes = 200.0 * static_cast<double>(args.vocab) / 150000.0;
     const double fixed = 45.0;
     uint32_t best = 0;
     double best_cost = 0.0;
-    for (uint32_t i = 0; i < 5u; ++i)
+    for (uint32_t i = 0; i < kClusterSizes; ++i)
     {
         const uint32_t size = 1u << i;
         const uint32_t resident = known.active[i] < static_cast<int>(ws.slots) ? static_cast<uint32_t>(known.active[i]) : ws.slots;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 
 #include "../../include/moe_b200_sampler.h"
@@ -175,16 +176,18 @@ cudaError_t launch_regroup_gather(const float* hidden, uint32_t token_count, uin
 constexpr int kMaxDevices = 64;
 struct SharedOptIn
 {
+    std::mutex guard; // held from the look at `bytes` until the attribute is set: nobody launches in between
     size_t bytes[kMaxDevices] = {};
 };
-// true when `shared_bytes` still has to be configured on `device`; records it as configured
+// true when `shared_bytes` still has to be configured on `device`; records it as configured (the caller holds the guard
+// and configures it)
 inline bool opt_in_needed(SharedOptIn& state, int device, size_t shared_bytes)
 {
     if (device < 0 || device >= kMaxDevices)
         return true; // untracked ordinal: configure on every launch
     if (state.bytes[device] >= shared_bytes)
         return false;
-    state.bytes[device] = shared_bytes; // racing host threads write the same value
+    state.bytes[device] = shared_bytes;
     return true;
 }
 template<typename Kernel>
@@ -194,12 +197,53 @@ cudaError_t opt_in_shared(SharedOptIn& state, Kernel kernel, size_t shared_bytes
     cudaError_t status = cudaGetDevice(&device);
     if (status != cudaSuccess)
         return status;
+    const std::lock_guard<std::mutex> lock(state.guard);
     if (!opt_in_needed(state, device, shared_bytes))
         return cudaSuccess;
     status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared_bytes));
     if (status != cudaSuccess && device >= 0 && device < kMaxDevices)
         state.bytes[device] = 0;
     return status;
+}
+
+// Clusters of 1, 2, 4, 8 and 16 CTAs of one kernel that a device holds at once; 0: none of that size.
+constexpr int kClusterSizes = 5;
+struct ClusterOccupancy
+{
+    int active[kClusterSizes] = {};
+};
+struct ClusterOccupancyTable
+{
+    std::mutex guard;
+    bool known[kMaxDevices] = {};
+    ClusterOccupancy found[kMaxDevices];
+};
+// query(size_index, &clusters) -> cudaError_t.  Asked once per device, unless a size up to the portable 8 was not
+// answered: then the call makes do with what it has (clusters of one CTA at least) and the next one asks again.
+template<typename Query>
+ClusterOccupancy cluster_occupancy(ClusterOccupancyTable& table, int device, Query query)
+{
+    const bool tracked = device >= 0 && device < kMaxDevices;
+    const std::lock_guard<std::mutex> lock(table.guard);
+    if (tracked && table.known[device])
+        return table.found[device];
+    ClusterOccupancy found;
+    bool answered = true;
+    for (int i = 0; i < kClusterSizes; ++i)
+    {
+        if (query(i, &found.active[i]) == cudaSuccess)
+            continue;
+        found.active[i] = 0;
+        answered = answered && (1 << i) > 8;
+    }
+    if (found.active[0] < 1)
+        found.active[0] = 1;
+    if (tracked && answered)
+    {
+        table.found[device] = found;
+        table.known[device] = true;
+    }
+    return found;
 }
 
 // Kernels are launched while the kernel before them in the stream may still run (programmatic stream serialization)

@@ -111,3 +111,19 @@ def test_shared_memory_opt_in_bookkeeping(tmp_path):
     subprocess.run([compiler, "-std=c++17", "-O1", f"-I{include}", str(root / "tests" / "cpp" / "opt_in_test.cpp"), "-o", str(target)], check=True)
     result = subprocess.run([str(target)], capture_output=True, text=True, timeout=60)
     assert result.returncode == 0, result.stdout + result.stderr
+
+
+def test_first_launches_of_several_threads(tmp_path):
+    """tests/cpp/opt_in_threads_test.cpp: a kernel's first launches from several host threads, with fakes for the runtime calls."""
+    import shutil
+    import subprocess
+    compiler = shutil.which("g++")
+    include = Path("/usr/local/cuda/include")
+    if compiler is None or not (include / "cuda_runtime.h").exists():
+        import pytest
+        pytest.skip("needs g++ and the CUDA headers")
+    target = tmp_path / "opt_in_threads_test"
+    subprocess.run([compiler, "-std=c++17", "-O1", "-pthread", f"-I{include}", str(ROOT / "tests" / "cpp" / "opt_in_threads_test.cpp"), "-o", str(target)],
+                   check=True)
+    result = subprocess.run([str(target)], capture_output=True, text=True, timeout=60)
+    assert result.returncode == 0, result.stdout + result.stderr
