@@ -196,8 +196,9 @@ int upload_rows(moe_sampler* sampler, cudaStream_t stream, uint32_t rows, const 
     return MOE_STATUS_OK;
 }
 
-// The exact kernel's per-slot sort scratch (16 bytes per vocabulary entry and
-// slot) is only needed by batches that contain rows without Top-K: it is
+// The exact kernels' scratch (16 bytes per vocabulary entry and slot; the
+// clusters and the one-CTA kernel behind them use the same slots one after the
+// other) is only needed by batches that contain rows without Top-K: it is
 // allocated when the first such batch arrives, not with the handle.
 int ensure_exact_scratch(moe_sampler* sampler, cudaStream_t stream)
 {
@@ -206,10 +207,7 @@ int ensure_exact_scratch(moe_sampler* sampler, cudaStream_t stream)
         return MOE_STATUS_OK;
     const size_t stride = (static_cast<size_t>(ws.max_vocab) + 3u) & ~static_cast<size_t>(3u);
     MOE_CUDA_CHECK(sampler, cudaStreamSynchronize(stream));
-    // one allocation: the sort scratch, then the clusters' items
-    const size_t sort_words = 4u * stride * ws.slots;
-    MOE_CUDA_CHECK(sampler, cudaMalloc(reinterpret_cast<void**>(&ws.sort_keys), sizeof(uint32_t) * (sort_words + 2u * (stride + 64u) * ws.slots)));
-    ws.exact_items = ws.sort_keys + sort_words;
+    MOE_CUDA_CHECK(sampler, cudaMalloc(reinterpret_cast<void**>(&ws.sort_keys), sizeof(uint32_t) * 4u * stride * ws.slots));
     return MOE_STATUS_OK;
 }
 

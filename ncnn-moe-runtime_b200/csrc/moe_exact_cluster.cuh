@@ -617,9 +617,9 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
     const uint32_t cluster_size = cluster.num_blocks();
     const uint32_t rank = cluster.block_rank();
     const float* row_pointer = row_logits<float>(a, row);
-    const uint32_t per = ((a.vocab + cluster_size - 1u) / cluster_size + 3u) & ~3u;
-    const uint32_t begin = min(a.vocab, rank * per);
-    const uint32_t end = min(a.vocab, begin + per);
+    const ClusterSlice slice = cluster_slice(a.vocab, cluster_size, rank);
+    const uint32_t begin = slice.begin;
+    const uint32_t end = slice.end;
     const uint32_t vectors = (end - begin + 3u) / 4u;
     outcome = RowOutcome{MOE_ROW_OK, -1, 0.0f, 0u, false};
 
@@ -1200,11 +1200,10 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
     wait_for_previous_kernel();
     const uint32_t pending = *ws.exact_count;
     const uint32_t slot_stride = (ws.max_vocab + 3u) & ~3u;
-    // the cluster's items (numerators, then group numbers), every CTA its slice; padded so that slices stay 16-byte aligned
+    // the cluster's items (numerators, then group numbers) in the slot of its number, every CTA its slice
     const uint32_t cluster_index = blockIdx.x / cluster_size;
-    const uint32_t item_stride = slot_stride + 4u * kMaxCluster;
-    uint32_t* items = ws.exact_items + static_cast<size_t>(cluster_index) * 2u * item_stride;
-    const uint32_t item_begin = rank * (((a.vocab + cluster_size - 1u) / cluster_size + 3u) & ~3u);
+    uint32_t* items = ws.sort_keys + static_cast<size_t>(cluster_index) * 4u * slot_stride;
+    const uint32_t item_begin = cluster_slice(a.vocab, cluster_size, rank).begin;
     cluster.sync(); // every CTA of the cluster runs before its shared memory is written to
     for (;;)
     {
@@ -1224,7 +1223,7 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
         RowOutcome outcome{MOE_ROW_OK, -1, 0.0f, 0u, false};
         if (p.top_k == 0 && a.kept_count == nullptr)
             handled = exact_row_cluster(a, row, p, reinterpret_cast<float*>(items) + item_begin,
-                                        reinterpret_cast<uint16_t*>(items + item_stride) + item_begin, cs, cluster, outcome);
+                                        reinterpret_cast<uint16_t*>(items + slot_stride) + item_begin, cs, cluster, outcome);
         if (rank == 0)
         {
             __syncthreads();

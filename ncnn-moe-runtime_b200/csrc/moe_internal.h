@@ -32,10 +32,9 @@ struct Workspace
     // rows the clusters left to the one-CTA kernel of the same call (with a mark in the high bit), and their number
     uint32_t* exact_deferred = nullptr;       // [max_rows]
     uint32_t* exact_deferred_count = nullptr; // [1]
-    // per-slot scratch of the exact kernel: (keys, index) pair 0 then pair 1,
-    // each array `max_vocab` rounded up to a multiple of 4 entries
+    // per-slot scratch of the exact kernels, stride = max_vocab rounded up to a multiple of 4 entries: two buffers of
+    // 64-bit items for the one-CTA kernel; the cluster kernel before it keeps its items there (see ClusterSlice)
     uint32_t* sort_keys = nullptr;     // [slots][4][stride]
-    uint32_t* exact_items = nullptr;   // [slots][2][stride + 64]: numerators and value groups of the row a cluster works on
     // publication slots of the streaming kernel when a row is cut into slices:
     // one per CTA, MOE_SLICE_SLOT_RECORDS records and a 4-word header each
     uint64_t* slice_records = nullptr; // [slice_slots][MOE_SLICE_SLOT_RECORDS]
@@ -46,6 +45,23 @@ struct Workspace
     uint32_t max_rows = 0;
     uint32_t max_vocab = 0;
 };
+
+// The part [begin, end) of a row that one CTA of a cluster owns.  Slices begin at multiples of four logits and their items
+// are written in whole groups of four, so a cluster's items end at the row's length rounded up to four: the numerators
+// (4 B) fill at most the first of a slot's four arrays, the value groups (2 B) at most half of the second.
+struct ClusterSlice
+{
+    uint32_t begin;
+    uint32_t end;
+};
+__host__ __device__ inline ClusterSlice cluster_slice(uint32_t vocab, uint32_t cluster_size, uint32_t rank)
+{
+    const uint32_t per = ((vocab + cluster_size - 1u) / cluster_size + 3u) & ~3u;
+    const uint64_t begin = static_cast<uint64_t>(rank) * per;
+    if (begin >= vocab)
+        return ClusterSlice{vocab, vocab}; // nothing left for it
+    return ClusterSlice{static_cast<uint32_t>(begin), vocab - static_cast<uint32_t>(begin) < per ? vocab : static_cast<uint32_t>(begin) + per};
+}
 
 struct SampleArgs
 {

@@ -113,8 +113,8 @@ def test_shared_memory_opt_in_bookkeeping(tmp_path):
     assert result.returncode == 0, result.stdout + result.stderr
 
 
-def test_first_launches_of_several_threads(tmp_path):
-    """tests/cpp/opt_in_threads_test.cpp: a kernel's first launches from several host threads, with fakes for the runtime calls."""
+
+def run_host_test(tmp_path, name):
     import shutil
     import subprocess
     compiler = shutil.which("g++")
@@ -122,8 +122,17 @@ def test_first_launches_of_several_threads(tmp_path):
     if compiler is None or not (include / "cuda_runtime.h").exists():
         import pytest
         pytest.skip("needs g++ and the CUDA headers")
-    target = tmp_path / "opt_in_threads_test"
-    subprocess.run([compiler, "-std=c++17", "-O1", "-pthread", f"-I{include}", str(ROOT / "tests" / "cpp" / "opt_in_threads_test.cpp"), "-o", str(target)],
-                   check=True)
+    target = tmp_path / name
+    subprocess.run([compiler, "-std=c++17", "-O1", "-pthread", f"-I{include}", str(ROOT / "tests" / "cpp" / f"{name}.cpp"), "-o", str(target)], check=True)
     result = subprocess.run([str(target)], capture_output=True, text=True, timeout=60)
     assert result.returncode == 0, result.stdout + result.stderr
+
+
+def test_first_launches_of_several_threads(tmp_path):
+    """tests/cpp/opt_in_threads_test.cpp: a kernel's first launches from several host threads, with fakes for the runtime calls."""
+    run_host_test(tmp_path, "opt_in_threads_test")
+
+
+def test_cluster_items_stay_inside_their_slot(tmp_path):
+    """tests/cpp/scratch_layout_test.cpp: how a cluster cuts a row and where it keeps its items."""
+    run_host_test(tmp_path, "scratch_layout_test")

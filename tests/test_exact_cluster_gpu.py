@@ -82,3 +82,44 @@ def test_infinities_and_nans(pkg, parity):
     for temperature in (1.0, 0.5):
         params = pkg.make_row_params(len(rows), seed=9, top_k=0, temperature=temperature, top_p=0.97)
         parity.check(logits, params)
+
+
+@pytest.mark.parametrize("stored", ["fp32", "bf16"])
+def test_scratch_of_the_first_batch_without_top_k(pkg, torch_cuda, stored):
+    """The first batch with a row without Top-K allocates 16 bytes per vocabulary entry and slot, whatever its logits' type."""
+    torch = torch_cuda
+    rows, vocab = 148, 201088
+    slots = min(rows, torch.cuda.get_device_properties(0).multi_processor_count)
+    logits = (3.0 * torch.randn((1, vocab), device="cuda")).to(torch.float32 if stored == "fp32" else torch.bfloat16)
+    warm = pkg.Sampler(max_rows=1, max_vocab=vocab)   # the kernels are loaded and have their stacks
+    warm.sample_batch(logits, pkg.make_row_params(1, seed=1, top_k=0))
+    torch.cuda.synchronize()
+    warm.close()
+    sampler = pkg.Sampler(max_rows=rows, max_vocab=vocab)
+    try:
+        out = sampler.sample_batch(logits, pkg.make_row_params(1, seed=1, top_k=50))
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        sampler.sample_batch(logits, pkg.make_row_params(1, seed=1, top_k=0), out=out)
+        torch.cuda.synchronize()
+        taken = before - torch.cuda.mem_get_info()[0]
+        assert 16 * vocab * slots <= taken <= 16 * vocab * slots + (8 << 20)
+    finally:
+        sampler.close()
+
+
+@pytest.mark.parametrize("vocab", [33, 4099, 20480])
+def test_handle_no_larger_than_the_row(pkg, parity, torch_cuda, vocab):
+    """Rows as long as the handle allows, every slot in use at once: neighbouring slots must not see each other's items."""
+    rng = np.random.default_rng(vocab)
+    rows = 160
+    logits = rng.uniform(-6.0, 6.0, (rows, vocab)).astype(np.float32)
+    params = pkg.make_row_params(rows, seed=4, top_k=0, temperature=rng.choice(np.array([1.0, 3.0], dtype=np.float32), rows), top_p=0.999)
+    sampler = pkg.Sampler(max_rows=rows, max_vocab=vocab)
+    try:
+        out = sampler.sample_batch(torch_cuda.from_numpy(logits).cuda(), params)
+        torch_cuda.cuda.synchronize()
+        want = parity.checker.sample_batch(logits, params["temperature"], params["top_k"], params["top_p"], params["min_p"], parity.uniforms(params))
+        np.testing.assert_array_equal(out["token"].cpu().numpy(), want["token"])
+    finally:
+        sampler.close()
