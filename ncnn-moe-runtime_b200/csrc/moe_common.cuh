@@ -105,11 +105,12 @@ __device__ __forceinline__ float scaled_offset(float logit, float temperature, f
 }
 
 // ---- streaming 128-bit loads ----------------------------------------------------
-// Logits are read exactly once: read-only path, no L1 allocation.
+// Logits are read exactly once: no L1 allocation.  Not the read-only path (ld.global.nc), which is defined for data that
+// nobody writes while the kernel runs: a kernel launched behind its producer may be resident while the producer writes.
 __device__ __forceinline__ uint4 load_stream_16(const void* pointer)
 {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(pointer));
     return v;

@@ -605,7 +605,8 @@ __global__ void __launch_bounds__(256) regroup_gather_kernel(const float* hidden
         const uint32_t vectors = columns / 4;
         const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         // vectors [c, end) of a route's row, by the lanes of a warp; the copies leave with a streaming store so that the
-        // hidden rows stay in L2
+        // hidden rows stay in L2.  Loads from L2, not through the read-only path: the kernel before this one may still
+        // have been writing the rows when this one became resident.
         const auto copy = [&](uint32_t route, uint32_t c, uint32_t end) {
             const uint32_t token = route_token[route];
             // a token index beyond the hidden matrix is never dereferenced: its row is zero-filled and the call flagged
@@ -619,13 +620,13 @@ __global__ void __launch_bounds__(256) regroup_gather_kernel(const float* hidden
                 float4 v[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
-                    v[u] = valid ? __ldg(source + c + 32u * u) : zero;
+                    v[u] = valid ? __ldcg(source + c + 32u * u) : zero;
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
                     __stcs(target + c + 32u * u, v[u]);
             }
             for (; c < end; c += 32)
-                __stcs(target + c, valid ? __ldg(source + c) : zero);
+                __stcs(target + c, valid ? __ldcg(source + c) : zero);
         };
         if (piece >= vectors)
         {

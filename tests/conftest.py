@@ -64,6 +64,22 @@ def sampler(pkg, torch_cuda):
     handle.close()
 
 
+@pytest.fixture(scope="session")
+def test_kernels():
+    """tests/cuda/kernels.cu, compiled beside its source when that is newer."""
+    import ctypes
+    import shutil
+    import subprocess
+    source = ROOT / "tests" / "cuda" / "kernels.cu"
+    target = source.with_name("libtest_kernels.so")
+    inputs = [source, ROOT / "ncnn-moe-runtime_b200" / "csrc" / "moe_common.cuh"]
+    if not target.exists() or any(path.stat().st_mtime > target.stat().st_mtime for path in inputs):
+        nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+        subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-shared", "-o", str(target),
+                        str(source)], check=True)
+    return ctypes.CDLL(str(target))
+
+
 class Parity:
     """Shared GPU-vs-oracle comparison used by the parity tests."""
 
