@@ -657,6 +657,12 @@ __global__ void __launch_bounds__(256) regroup_gather_kernel(const float* hidden
     }
 }
 
+// Whether one launch serves the call.  It uses none of the scratch in RouterArgs.
+bool in_one_launch(uint32_t token_count, const moe_router_options& options)
+{
+    return token_count <= kFewTokens && options.expert_count <= kNarrowExperts && options.top_k <= kNarrowTopK;
+}
+
 } // namespace
 
 cudaError_t launch_router_dispatch_kernels(const RouterArgs& caller_args, uint32_t* expert_counts, uint32_t* scan_done, unsigned long long* error_word,
@@ -664,7 +670,7 @@ cudaError_t launch_router_dispatch_kernels(const RouterArgs& caller_args, uint32
 {
     RouterArgs args = caller_args;
     const uint32_t experts = args.options.expert_count;
-    if (args.token_count <= kFewTokens && experts <= kNarrowExperts && args.options.top_k <= kNarrowTopK)
+    if (in_one_launch(args.token_count, args.options))
     {
         const size_t few_bytes = few_shared_bytes(experts, args.options.top_k);
         static SharedOptIn few_opt_in;
@@ -817,12 +823,15 @@ extern "C" int moe_router_dispatch_static(void* stream_handle, const float* rout
     StaticRouterScratch* scratch = static_cast<StaticRouterScratch*>(g_router_static_address[device]);
     cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
 
-    router_static_reset_kernel<<<1, 1, 0, stream>>>(scratch);
-    status = cudaGetLastError();
-    if (status != cudaSuccess)
+    if (!in_one_launch(token_count, *options))
     {
-        describe(error_text, error_capacity, cudaGetErrorString(status));
-        return MOE_STATUS_CUDA_ERROR;
+        router_static_reset_kernel<<<1, 1, 0, stream>>>(scratch);
+        status = cudaGetLastError();
+        if (status != cudaSuccess)
+        {
+            describe(error_text, error_capacity, cudaGetErrorString(status));
+            return MOE_STATUS_CUDA_ERROR;
+        }
     }
     RouterArgs args = {};
     args.logits = router_logits;
@@ -844,6 +853,3 @@ extern "C" int moe_router_dispatch_static(void* stream_handle, const float* rout
     }
     return MOE_STATUS_OK;
 }
-
-namespace moe {
-} // namespace moe

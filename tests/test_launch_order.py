@@ -89,3 +89,69 @@ def test_other_kernels_behind_a_producer_that_lets_them_start_early(pkg, torch_c
             plan = sampler.router_dispatch(x, 4)
             return [plan.expert_offsets, plan.route_token, plan.route_rank, plan.route_weight, plan.status]
         check(versions(tokens, 96), dispatch)
+
+
+class Captured:
+    """The launches of `call` on a stream of its own as a graph: how many kernels, and another run of them."""
+
+    def __init__(self, torch, call):
+        from cuda.bindings import runtime
+        self.runtime, self.torch, self.stream = runtime, torch, torch.cuda.Stream()
+        self.check(runtime.cudaStreamBeginCapture(self.stream.cuda_stream, runtime.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal))
+        try:
+            call(self.stream.cuda_stream)
+        finally:
+            self.graph = self.check(runtime.cudaStreamEndCapture(self.stream.cuda_stream))
+        count = self.check(runtime.cudaGraphGetNodes(self.graph, 0))[1]
+        nodes = self.check(runtime.cudaGraphGetNodes(self.graph, count))[0]
+        kinds = [self.check(runtime.cudaGraphNodeGetType(node)) for node in nodes]
+        self.kernels = sum(kind == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for kind in kinds)
+        self.nodes = len(kinds)
+        self.executable = self.check(runtime.cudaGraphInstantiate(self.graph, 0))
+
+    def check(self, result):
+        assert int(result[0]) == 0, result[0]
+        return result[1] if len(result) == 2 else result[1:]
+
+    def run(self):
+        self.check(self.runtime.cudaGraphLaunch(self.executable, self.stream.cuda_stream))
+        self.torch.cuda.synchronize()
+
+    def close(self):
+        self.runtime.cudaGraphExecDestroy(self.executable)
+        self.runtime.cudaGraphDestroy(self.graph)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,experts,top_k,launches", [(32, 128, 4, 1), (128, 1024, 16, 1), (129, 64, 4, 4), (4, 1025, 2, 4), (4, 64, 17, 4)])
+def test_static_router_launches_what_it_needs(pkg, sampler, torch_cuda, tokens, experts, top_k, launches):
+    """One launch for a few tokens; the three launches over the fixed scratch follow a reset of its counters."""
+    torch = torch_cuda
+    generator = torch.Generator(device="cuda").manual_seed(tokens)
+    logits = torch.randn((tokens, experts), generator=generator, device="cuda")
+    want = sampler.router_dispatch(logits, top_k)
+    torch.cuda.synchronize()
+    got = pkg.DispatchPlan(*[torch.empty_like(t) for t in (want.expert_offsets, want.route_token, want.route_rank, want.route_weight, want.status)])
+    options = pkg.RouterOptions(experts, top_k, pkg.ROUTER_SOFTMAX, 1, 1.0, pkg.ROUTER_FLAG_NORMALIZE_TOPK, None, None)
+
+    def dispatch(stream):
+        message = C.create_string_buffer(256)
+        pointers = [C.c_void_p(t.data_ptr()) for t in (logits, got.expert_offsets, got.route_token, got.route_rank, got.route_weight, got.status)]
+        code = pkg.library().moe_router_dispatch_static(C.c_void_p(stream), pointers[0], tokens, C.byref(options), *pointers[1:], message, 256)
+        assert code == 0, message.value
+
+    dispatch(torch.cuda.current_stream().cuda_stream)   # the scratch's address is looked up
+    torch.cuda.synchronize()
+    captured = Captured(torch, dispatch)
+    try:
+        assert captured.nodes == captured.kernels == launches
+        for _ in range(2):
+            for t in (got.expert_offsets, got.route_token, got.route_rank):
+                t.fill_(-1)
+            torch.cuda.synchronize()
+            captured.run()
+            for g, w in zip((got.expert_offsets, got.route_token, got.route_rank, got.route_weight, got.status),
+                            (want.expert_offsets, want.route_token, want.route_rank, want.route_weight, want.status)):
+                assert torch.equal(g, w)
+    finally:
+        captured.close()
