@@ -104,6 +104,17 @@ __device__ __forceinline__ float scaled_offset(float logit, float temperature, f
     return __fsub_rn(__fdiv_rn(logit, temperature), peak);
 }
 
+// a / b rounded to nearest, with r = 1 / b rounded to nearest: two Newton corrections of the quotient
+// with exact remainders (P. Markstein, IBM J. Res. Dev. 34, 1990: from a quotient within one unit in the
+// last place the last correction gives the correctly rounded one).  The remainder a - q * b is a multiple of
+// 2^(exponent of a - 47), so it is exact, and the quotient normal, for a >= 2^-100 and b in [2^-24, 2^25).
+__device__ __forceinline__ float divide_by(float a, float b, float r)
+{
+    float q = __fmul_rn(a, r);
+    q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
 // ---- streaming 128-bit loads ----------------------------------------------------
 // Logits are read exactly once: no L1 allocation.  Not the read-only path (ld.global.nc), which is defined for data that
 // nobody writes while the kernel runs: a kernel launched behind its producer may be resident while the producer writes.

@@ -365,17 +365,6 @@ __device__ __noinline__ void guess_exponents(ClusterShared& cs, uint32_t first_g
     __syncthreads();
 }
 
-// a / b rounded to nearest, with r = 1 / b rounded to nearest: two Newton corrections of the quotient
-// with exact remainders (P. Markstein, IBM J. Res. Dev. 34, 1990: from a quotient within one unit in the
-// last place the last correction gives the correctly rounded one).  a and b are far from the ends of
-// the exponent range here: a >= 2^-50, b between 2^-24 and 2^24.
-__device__ __forceinline__ float divide_by(float a, float b, float r)
-{
-    float q = __fmul_rn(a, r);
-    q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
-    return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
-}
-
 // Adds the peers' counters of this CTA's groups to its own (the tie bits are joined).  Sixteen bytes per
 // remote load, at most four loads per thread, all of them in flight together.
 __device__ __forceinline__ void reduce_table(ClusterShared& cs, cg::cluster_group& cluster, uint32_t owned_begin, uint32_t owned)
@@ -496,6 +485,9 @@ __device__ __forceinline__ void add_steps(const StepArgs& s, ClusterShared& cs, 
         {
             active[u] = any && g[u] - s.head_end <= active_range; // dead items have the largest group number
             float value = x[u];
+            // For numerators below the range of divide_by (a peak of 1e7 temperatures and more widens the live window to
+            // them) the quotient may be off in its last bits: it is below 2^-70 then, the accumulators start above
+            // 2^-25, so the item takes no step whatever they are, in or out of the Min-P list.
             if (kSum >= 1)
             {
                 value = divide_by(value, s.total, s.total_reciprocal);

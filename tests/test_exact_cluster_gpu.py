@@ -1,6 +1,8 @@
 """fp32 rows without Top-K that a thread-block cluster finishes: every cluster size (the batch size chooses it), every
 way a sum can end (in the head, inside a literal group, never), and the shapes the clusters leave to single CTAs.
 Tokens and probability bits are compared with the oracle, so no tolerance applies."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -123,3 +125,43 @@ def test_handle_no_larger_than_the_row(pkg, parity, torch_cuda, vocab):
         np.testing.assert_array_equal(out["token"].cpu().numpy(), want["token"])
     finally:
         sampler.close()
+
+
+def _compare_divisions(test_kernels, seed, a_exponents, b_exponents):
+    mismatches, largest = C.c_ulonglong(), C.c_float()
+    code = test_kernels.test_compare_divisions(C.c_uint64(seed), C.c_uint32(1184), C.c_uint32(1024), *[C.c_int(e) for e in (*a_exponents, *b_exponents)],
+                                               C.byref(mismatches), C.byref(largest))
+    assert code == 0
+    return mismatches.value, largest.value
+
+
+@pytest.mark.parametrize("a_exponents,b_exponents", [((-27, 0), (0, 17)), ((-45, 0), (-18, 0)), ((-100, 1), (-24, 24)), ((-100, -90), (20, 24))])
+def test_division_by_a_reciprocal(torch_cuda, test_kernels, a_exponents, b_exponents):
+    """The item passes divide by the two normalisers with a reciprocal and two corrections: every quotient of seeded pairs (a
+    quarter of the mantissas next to a power of two or to the middle) is the division's, over the operands of ordinary rows (the
+    first two) and over the whole range the function is stated for."""
+    assert _compare_divisions(test_kernels, 1 - a_exponents[0], a_exponents, b_exponents)[0] == 0
+
+
+def test_division_of_numerators_below_the_range(torch_cuda, test_kernels):
+    """Numerators below 2^-100, zero and denormal ones among them, give finite quotients below 2^-70: no step in any accumulator."""
+    _, largest = _compare_divisions(test_kernels, 5, (-127, -101), (-24, 24))
+    assert largest < 2.0 ** -70
+
+
+def test_peaks_far_above_the_temperature(pkg, parity):
+    """A peak of 1e6 to 1e8 temperatures: the logits lie on a coarse grid, the live window is wider and holds numerators that
+    are tiny or zero."""
+    rng = np.random.default_rng(17)
+    vocab = 60001
+    rows = []
+    for scale in (1.0e6, 1.0e7, 1.0e8):
+        base = np.float32(scale)
+        rows.append(base - np.abs(rng.standard_normal(vocab)).astype(np.float32) * np.float32(40.0 + scale * 2.0e-6))
+        rows.append(base - rng.uniform(0.0, 3.0e-6 * scale, vocab).astype(np.float32))
+    logits = np.stack(rows).astype(np.float32)
+    for temperature, min_p in ((1.0, 0.0), (4.0, 1e-30), (0.5, 1e-4)):
+        params = pkg.make_row_params(len(rows), seed=6, top_k=0, temperature=temperature, top_p=0.9999, min_p=min_p)
+        for step in range(2):
+            params["step"] = step
+            parity.check(logits, params)
