@@ -191,10 +191,13 @@ def test_router_errors(sampler, pkg):
     assert sampler.router_dispatch_host(logits, 4, 8, 2).status == 0
 
 
-@pytest.mark.parametrize("columns,routes", [(4, 444 * 33 + 5), (4, 445), (36, 444 * 32), (1024, 444 * 34 + 1), (4100, 1000), (8, 1), (6, 100)])
+# (4096, 6000): 24000 pieces of 4 KiB for the grid's 18944 warps; (1028, 25000): more than 96 MiB, whole rows, more than warps
+@pytest.mark.parametrize("columns,routes", [(4, 444 * 33 + 5), (4, 445), (36, 444 * 32), (1024, 444 * 34 + 1), (4100, 1000), (8, 1), (6, 100),
+                                            (4096, 6000), (1028, 25000), (6, 20000), (4, 20000)])
 def test_gather_moves_rows_in_pieces(sampler, torch_cuda, columns, routes):
-    """Row lengths from one 16-byte vector to several pieces, and as many pieces per warp as make its groups of ids and its
-    slots wrap; ids outside the matrix (their rows become zero, the call is flagged) between the others."""
+    """Row lengths from one 16-byte vector to several 4 KiB pieces and rows without vectors; calls of a few warps (small
+    blocks), of more pieces than warps (a warp takes a second one) and of whole rows; ids outside the matrix (their rows
+    become zero, the call is flagged) between the others."""
     torch = torch_cuda
     generator = torch.Generator(device="cuda").manual_seed(columns + routes)
     tokens = 97
