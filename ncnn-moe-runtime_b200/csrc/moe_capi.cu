@@ -34,9 +34,8 @@ struct moe_sampler
     bool overlap_launches = false;
     bool resident_has_stops = false;
 
-    // per-row records of moe_sample_tokens: page-locked host memory, and the address the kernels write it through
+    // per-row records of moe_sample_tokens: page-locked host memory the kernels write through (allocated by its first call)
     moe_sampled_row* sampled_host = nullptr;
-    moe_sampled_row* sampled_mapped = nullptr;
 
     // staging for the host-buffer entry points
     void* logits_dev = nullptr;
@@ -292,10 +291,6 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
     allocate(reinterpret_cast<void**>(&sampler->probability_dev), sizeof(float) * max_rows);
     allocate(reinterpret_cast<void**>(&sampler->flags_dev), sizeof(uint32_t) * max_rows);
     allocate(reinterpret_cast<void**>(&sampler->status_dev), sizeof(int32_t) * max_rows);
-    if (status == cudaSuccess)
-        status = cudaHostAlloc(reinterpret_cast<void**>(&sampler->sampled_host), sizeof(moe_sampled_row) * max_rows, cudaHostAllocMapped);
-    if (status == cudaSuccess)
-        status = cudaHostGetDevicePointer(reinterpret_cast<void**>(&sampler->sampled_mapped), sampler->sampled_host, 0);
     allocate(reinterpret_cast<void**>(&sampler->router_error), sizeof(unsigned long long));
     allocate(reinterpret_cast<void**>(&sampler->router_scan_done), sizeof(uint32_t));
     allocate(reinterpret_cast<void**>(&sampler->gather_status), sizeof(int32_t));
@@ -693,10 +688,14 @@ int moe_sample_tokens(moe_sampler* sampler, void* stream_handle, const void* log
         return fail(sampler, MOE_STATUS_INVALID_ARGUMENT, "logits and results must not be null");
     cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
     DeviceGuard guard(sampler->device);
+    if (sampler->sampled_host == nullptr)
+        MOE_CUDA_CHECK(sampler, cudaHostAlloc(reinterpret_cast<void**>(&sampler->sampled_host), sizeof(moe_sampled_row) * sampler->max_rows, cudaHostAllocMapped));
     // The kernel that finishes a row stores its 16-byte record straight into host memory: a packing kernel and a
     // device-to-host copy behind the sampler cost another two submissions and about 7 us per call.
+    moe_sampled_row* records = nullptr;
+    MOE_CUDA_CHECK(sampler, cudaHostGetDevicePointer(reinterpret_cast<void**>(&records), sampler->sampled_host, 0));
     const moe_sample_outputs outputs = {};
-    const int status = sample_rows(sampler, stream, logits, dtype, rows, vocab, row_stride, params, step_offset, stop_offsets, stop_tokens, &outputs, sampler->sampled_mapped);
+    const int status = sample_rows(sampler, stream, logits, dtype, rows, vocab, row_stride, params, step_offset, stop_offsets, stop_tokens, &outputs, records);
     if (status != MOE_STATUS_OK)
         return status;
     MOE_CUDA_CHECK(sampler, cudaStreamSynchronize(stream));

@@ -155,28 +155,3 @@ def test_static_router_launches_what_it_needs(pkg, sampler, torch_cuda, tokens, 
                 assert torch.equal(g, w)
     finally:
         captured.close()
-
-
-@pytest.mark.gpu
-def test_first_tokens_while_another_stream_is_captured(pkg, torch_cuda):
-    """A global-mode capture forbids allocations to its thread: a handle's first moe_sample_tokens call makes none."""
-    from cuda.bindings import runtime
-    torch = torch_cuda
-    rows, vocab = 4, 5000
-    logits = torch.randn((rows, vocab), device="cuda")
-    sampler = pkg.Sampler(max_rows=rows, max_vocab=vocab)
-    captured, other = torch.cuda.Stream(), torch.cuda.Stream()
-    results = np.zeros(rows, dtype=pkg.SAMPLED_ROW_DTYPE)
-    try:
-        want = sampler.sample_batch(logits, pkg.make_row_params(rows, seed=2, top_k=20))
-        torch.cuda.synchronize()
-        assert int(runtime.cudaStreamBeginCapture(captured.cuda_stream, runtime.cudaStreamCaptureMode.cudaStreamCaptureModeGlobal)[0]) == 0
-        try:
-            sampler.sample_tokens(logits, None, stream=other.cuda_stream, results=results)
-        finally:
-            ended = runtime.cudaStreamEndCapture(captured.cuda_stream)
-        assert int(ended[0]) == 0
-        runtime.cudaGraphDestroy(ended[1])
-        np.testing.assert_array_equal(results["token"], want["token"].cpu().numpy())
-    finally:
-        sampler.close()
