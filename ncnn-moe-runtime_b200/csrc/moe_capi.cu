@@ -278,7 +278,7 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
             status = cudaMalloc(pointer, bytes);
     };
     uint32_t* counters = nullptr;
-    allocate(reinterpret_cast<void**>(&counters), 4 * sizeof(uint32_t));
+    allocate(reinterpret_cast<void**>(&counters), 8 * sizeof(uint32_t));
     allocate(reinterpret_cast<void**>(&ws.exact_deferred), sizeof(uint32_t) * max_rows);
     allocate(reinterpret_cast<void**>(&ws.exact_rows), sizeof(uint32_t) * max_rows);
     ws.slice_slots = static_cast<uint32_t>(sampler->sm_count) * 6u * 2u + 64u;
@@ -296,7 +296,7 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
     allocate(reinterpret_cast<void**>(&sampler->gather_status), sizeof(int32_t));
     allocate(reinterpret_cast<void**>(&sampler->router_status_dev), sizeof(int32_t));
     if (status == cudaSuccess)
-        status = cudaMemset(counters, 0, 4 * sizeof(uint32_t));
+        status = cudaMemset(counters, 0, 8 * sizeof(uint32_t));
     if (status == cudaSuccess)
         status = cudaMemset(ws.row_arrivals, 0, sizeof(uint32_t) * max_rows);
     if (status == cudaSuccess)
@@ -313,6 +313,7 @@ int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sa
     ws.exact_done = counters != nullptr ? counters + 1 : nullptr;
     ws.exact_next = counters != nullptr ? counters + 2 : nullptr;
     ws.exact_deferred_count = counters != nullptr ? counters + 3 : nullptr;
+    ws.cluster_counts = counters != nullptr ? counters + 4 : nullptr;
     if (status != cudaSuccess)
     {
         moe_sampler_destroy(sampler);
@@ -499,6 +500,26 @@ int moe_sample_batch_ex(moe_sampler* sampler, void* stream_handle, const void* l
                         const moe_sample_outputs* outputs)
 {
     return sample_rows(sampler, stream_handle, logits, dtype, rows, vocab, row_stride, params, step_offset, stop_offsets, stop_tokens, outputs, nullptr);
+}
+
+int moe_internal_set_cluster_ctas(moe_sampler* sampler, uint32_t ctas)
+{
+    if (sampler == nullptr || ctas > 16u || (ctas & (ctas - 1u)) != 0u)
+        return MOE_STATUS_INVALID_ARGUMENT;
+    sampler->ws.cluster_ctas = ctas;
+    return MOE_STATUS_OK;
+}
+
+int moe_internal_cluster_counts(moe_sampler* sampler, void* stream_handle, uint32_t* counts)
+{
+    if (sampler == nullptr || counts == nullptr)
+        return MOE_STATUS_INVALID_ARGUMENT;
+    DeviceGuard guard(sampler->device);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_handle);
+    MOE_CUDA_CHECK(sampler, cudaMemcpyAsync(counts, sampler->ws.cluster_counts, sizeof(uint32_t) * 4u, cudaMemcpyDeviceToHost, stream));
+    MOE_CUDA_CHECK(sampler, cudaMemsetAsync(sampler->ws.cluster_counts, 0, sizeof(uint32_t) * 4u, stream));
+    MOE_CUDA_CHECK(sampler, cudaStreamSynchronize(stream));
+    return MOE_STATUS_OK;
 }
 
 int moe_speculative_verify_batch(moe_sampler* sampler, void* stream_handle, const void* target_logits, const void* draft_logits, int dtype,

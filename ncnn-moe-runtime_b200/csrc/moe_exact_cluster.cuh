@@ -29,8 +29,6 @@
 
 #include <cooperative_groups.h>
 
-#include <cstdlib>
-
 namespace moe {
 
 namespace {
@@ -138,6 +136,7 @@ struct alignas(16) ClusterShared
     Jump jump[kMaxGuesses];
     SumState state;
     SumState next_state; // rank 0: under construction
+    uint32_t counts[4];  // Workspace::cluster_counts of this cluster
 };
 constexpr size_t kClusterSharedBytes = sizeof(ClusterShared);
 
@@ -931,8 +930,8 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
             const uint32_t literal_groups = first_cta.literal_count;
             const uint32_t literal_items = first_cta.literal_items;
             CL_MARK(22);
-            CL_COUNT(28, literal_groups);
-            CL_COUNT(29, 1);
+            CL_COUNT(27, literal_groups);
+            CL_COUNT(28, 1);
             // exponents of my groups behind `from`, taken from the accumulators found
             const auto publish_exponents = [&](uint32_t from) {
                 running = first_running;
@@ -955,6 +954,8 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                 // the guess was too far off: repeat with the exponents of the accumulators just found
                 publish_exponents(0u);
                 jump_count = 0;
+                if (tid == 0)
+                    ++cs.counts[3];
                 cluster.sync();
                 continue;
             }
@@ -993,7 +994,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
             cluster.sync();
 
             CL_MARK(23);
-            CL_COUNT(30, cs.item_count);
+            CL_COUNT(29, cs.item_count);
             // ---- rank 0 walks them ----------------------------------------------------------------
             if (rank == 0)
             {
@@ -1160,7 +1161,10 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
             if (guess + 1 == kMaxGuesses)
                 return false;
             if (tid == 0)
+            {
                 cs.jump[jump_count] = Jump{cs.state.repeat_group, cs.state.repeat_delta};
+                ++cs.counts[2];
+            }
             ++jump_count;
             __syncthreads();
             publish_exponents(cs.state.repeat_group);
@@ -1196,6 +1200,8 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
     const uint32_t cluster_index = blockIdx.x / cluster_size;
     uint32_t* items = ws.sort_keys + static_cast<size_t>(cluster_index) * 4u * slot_stride;
     const uint32_t item_begin = cluster_slice(a.vocab, cluster_size, rank).begin;
+    if (tid < 4u)
+        cs.counts[tid] = 0;
     cluster.sync(); // every CTA of the cluster runs before its shared memory is written to
     for (;;)
     {
@@ -1221,9 +1227,11 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
             __syncthreads();
             if (!handled)
             {
-                CL_COUNT(27, 1);
                 if (tid == 0)
+                {
                     ws.exact_deferred[atomicAdd(ws.exact_deferred_count, 1u)] = row | (outcome.defer ? kBf16ValuedRow : 0u);
+                    ++cs.counts[1];
+                }
             }
             else
             {
@@ -1235,11 +1243,14 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
                     if (outcome.status == MOE_ROW_OK && is_stop_token(a.stop_offsets, a.stop_tokens, row, outcome.token))
                         outcome.flags |= MOE_ROW_FLAG_STOP_TOKEN;
                     write_row_result(a, row, outcome.token, outcome.probability, outcome.flags, outcome.status);
+                    ++cs.counts[0];
                 }
             }
         }
         cluster.sync();
     }
+    if (rank == 0 && tid < 4u && cs.counts[tid] != 0u)
+        atomicAdd(ws.cluster_counts + tid, cs.counts[tid]);
     if (tid == 0)
     {
         __threadfence();
@@ -1309,10 +1320,9 @@ cudaError_t launch_sample_exact_cluster(const SampleArgs& args, const Workspace&
             best_cost = cost;
         }
     }
-#ifdef MOE_PHASE_TIMERS
-    if (const char* forced = std::getenv("MOE_B200_EXACT_CLUSTER"))
-        best = static_cast<uint32_t>(std::atoi(forced));
-#endif
+    for (uint32_t i = 0; i < kClusterSizes; ++i)
+        if (ws.cluster_ctas == 1u << i && known.active[i] > 0)
+            best = i;
     const uint32_t size = 1u << best;
     const uint32_t resident = known.active[best] < static_cast<int>(ws.slots) ? static_cast<uint32_t>(known.active[best]) : ws.slots;
     const uint32_t clusters = rows < resident ? rows : resident;

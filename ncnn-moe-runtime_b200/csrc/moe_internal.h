@@ -32,6 +32,10 @@ struct Workspace
     // rows the clusters left to the one-CTA kernel of the same call (with a mark in the high bit), and their number
     uint32_t* exact_deferred = nullptr;       // [max_rows]
     uint32_t* exact_deferred_count = nullptr; // [1]
+    // what the clusters did since it was last read, for tests (a row they leave has the same result): rows finished, rows
+    // left, sums repeated with a corrected accumulator, sums repeated with better exponents
+    uint32_t* cluster_counts = nullptr; // [4]
+    uint32_t cluster_ctas = 0;          // CTAs per row; 0: chosen by the launcher
     // per-slot scratch of the exact kernels, stride = max_vocab rounded up to a multiple of 4 entries: two buffers of
     // 64-bit items for the one-CTA kernel; the cluster kernel before it keeps its items there (see ClusterSlice)
     uint32_t* sort_keys = nullptr;     // [slots][4][stride]
@@ -294,3 +298,9 @@ cudaError_t launch_indexer_topk(const float* scores, uint32_t rows, uint32_t cou
 uint32_t choose_splits(uint32_t rows, uint32_t vocab, int dtype, int sm_count, uint32_t slice_slots, bool large_top_k, bool overlapped);
 
 } // namespace moe
+
+// ---- for tests; not part of the ABI ----
+// Fixes the CTAs per row of the handle's clusters (1, 2, 4, 8 or 16; 0: chosen by the launcher).
+extern "C" int moe_internal_set_cluster_ctas(moe_sampler* sampler, uint32_t ctas);
+// Synchronises `stream`, copies Workspace::cluster_counts to the host and clears them.
+extern "C" int moe_internal_cluster_counts(moe_sampler* sampler, void* stream, uint32_t* counts);

@@ -1,5 +1,6 @@
-"""fp32 rows without Top-K that a thread-block cluster finishes: every cluster size (the batch size chooses it), every
-way a sum can end (in the head, inside a literal group, never), and the shapes the clusters leave to single CTAs.
+"""fp32 rows without Top-K that a thread-block cluster finishes: every cluster size (fixed, and chosen from the batch size),
+every way a sum can end (in the head, inside a literal group, never), sums that are repeated, and the rows the clusters
+leave to single CTAs.  A row that is left has the same result, so the tests also look at what the clusters counted.
 Tokens and probability bits are compared with the oracle, so no tolerance applies."""
 import ctypes as C
 
@@ -23,6 +24,98 @@ def _rows(rng, vocab):
     masked[rng.random(vocab) < 0.5] = -np.inf
     rows.append(masked)
     return np.stack(rows).astype(np.float32)
+
+
+class Clusters:
+    """The cluster size of a handle, and what its clusters have done since the last look."""
+
+    def __init__(self, pkg, torch, sampler, size):
+        self.library, self.torch, self.sampler = pkg.library(), torch, sampler
+        assert self.library.moe_internal_set_cluster_ctas(sampler._handle, size) == 0
+
+    def counts(self):
+        words = (C.c_uint32 * 4)()
+        assert self.library.moe_internal_cluster_counts(self.sampler._handle, C.c_void_p(self.torch.cuda.current_stream().cuda_stream), words) == 0
+        return dict(zip(("rows", "left", "repeats", "refinements"), words))
+
+    def __enter__(self):
+        self.counts()
+        return self
+
+    def __exit__(self, *_):
+        assert self.library.moe_internal_set_cluster_ctas(self.sampler._handle, 0) == 0
+
+
+@pytest.mark.parametrize("size", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("vocab", [2600, 40001, 151936])
+def test_ordinary_rows_are_finished_by_their_cluster(pkg, parity, torch_cuda, size, vocab):
+    """Ordinary rows with whole vocabularies alive (top_p = 0.5: the bound is the end of a binade): none is left."""
+    rng = np.random.default_rng(vocab)
+    rows = []
+    for _ in range(2):
+        normal = rng.standard_normal(vocab).astype(np.float32)
+        rows += [normal, 2.0 * normal, rng.uniform(-4.0, 4.0, vocab), 1000.0 + 3.0 * normal, -np.abs(normal) - 50.0]
+    logits = np.stack(rows).astype(np.float32)
+    params = pkg.make_row_params(len(rows), seed=size, top_k=0, temperature=3.0, top_p=np.array([0.5, 0.25, 0.95, 1.0, 0.999] * 2, dtype=np.float32))
+    with Clusters(pkg, torch_cuda, parity.sampler, size) as clusters:
+        for step in range(2):
+            params["step"] = step
+            parity.check(logits, params)
+        counts = clusters.counts()
+    assert counts["rows"] == 2 * len(rows) and counts["left"] == 0
+
+
+@pytest.mark.parametrize("size", [1, 2, 4, 8, 16])
+def test_sums_that_are_repeated(pkg, parity, torch_cuda, size):
+    """top_p = 1: the nucleus sum ends within ulps of its bound, where groups are literal in large numbers (a guess is refined)
+    and ties move the accumulator off the scanned one (the sum is repeated with the correction).  Both happen here."""
+    rng = np.random.default_rng(2)
+    vocab = 40001
+    logits = np.stack([-np.abs(3.0 * rng.standard_normal(vocab)) - 50.0 for _ in range(16)] +
+                      [-rng.exponential(2.0, vocab) for _ in range(16)]).astype(np.float32)
+    params = pkg.make_row_params(len(logits), seed=3, top_k=0, top_p=1.0)
+    with Clusters(pkg, torch_cuda, parity.sampler, size) as clusters:
+        for step in range(2):
+            params["step"] = step
+            parity.check(logits, params)
+        counts = clusters.counts()
+    assert counts["rows"] + counts["left"] == 2 * len(logits) and counts["rows"] > len(logits)
+    assert counts["repeats"] > 0 and counts["refinements"] > 0
+
+
+@pytest.mark.parametrize("size", [1, 4, 16])
+def test_rows_that_are_left(pkg, parity, torch_cuda, size):
+    """Rows of bf16 values, rows with more equal logits than a group holds, and rows with a Top-K above the streaming limit
+    are left to the one-CTA kernel; ordinary rows of the same batch are not."""
+    rng = np.random.default_rng(9)
+    vocab = 40001
+    normal = (3.0 * rng.standard_normal((4, vocab))).astype(np.float32)
+    widened = ((normal[1].view(np.uint32) >> 16) << 16).view(np.float32)
+    filled = normal[2].copy()
+    filled[-300:] = np.float32(0.1)
+    logits = np.stack([normal[0], widened, filled, normal[3]])
+    params = pkg.make_row_params(4, seed=1, top_k=np.array([0, 0, 0, 1500], dtype=np.uint32), temperature=1.5, top_p=0.99)
+    with Clusters(pkg, torch_cuda, parity.sampler, size) as clusters:
+        parity.check(logits, params)
+        counts = clusters.counts()
+    assert counts["rows"] == 1 and counts["left"] == 3
+
+
+@pytest.mark.parametrize("size", [1, 2, 16])
+def test_rows_of_odd_strides(pkg, parity, torch_cuda, size):
+    """Rows that begin at every 16-byte phase: slices that are read by vectors and slices that are not."""
+    rng = np.random.default_rng(6)
+    vocab, rows = 20003, 8
+    logits = (2.0 * rng.standard_normal((rows, vocab))).astype(np.float32)
+    wide = torch_cuda.zeros((rows, vocab + 2), device="cuda")   # a stride of 20005 logits
+    wide[:, :vocab] = torch_cuda.from_numpy(logits)
+    params = pkg.make_row_params(rows, seed=5, top_k=0, temperature=2.0, top_p=0.98)
+    with Clusters(pkg, torch_cuda, parity.sampler, size) as clusters:
+        out = parity.sampler.sample_batch(wide, params, vocab=vocab)
+        counts = clusters.counts()
+    assert counts["rows"] == rows and counts["left"] == 0
+    want = parity.checker.sample_batch(logits, params["temperature"], params["top_k"], params["top_p"], params["min_p"], parity.uniforms(params))
+    np.testing.assert_array_equal(out["token"].cpu().numpy(), want["token"])
 
 
 @pytest.mark.parametrize("copies", [1, 2, 4, 9, 20])

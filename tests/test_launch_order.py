@@ -155,3 +155,130 @@ def test_static_router_launches_what_it_needs(pkg, sampler, torch_cuda, tokens, 
                 assert torch.equal(g, w)
     finally:
         captured.close()
+
+
+class Calls:
+    """One call of every device-buffer entry point with resident parameters, into outputs of its own: kernels per call, the call,
+    and the tensors it writes."""
+
+    def __init__(self, pkg, torch, overlap=False):
+        generator = torch.Generator(device="cuda").manual_seed(11)
+
+        def normal(*shape):
+            return torch.randn(shape, generator=generator, device="cuda")
+
+        self.handles = {}
+        self.entries = {}
+
+        def sampling(name, launches, logits, **options):
+            rows, vocab = logits.shape
+            handle = self.handles[name] = pkg.Sampler(max_rows=rows, max_vocab=vocab)
+            handle.set_overlap(overlap)
+            out = handle.sample_batch(logits, pkg.make_row_params(rows, seed=5, **options))
+            self.entries[name] = (launches, lambda stream: handle.sample_batch(logits, None, stream=stream, out=out), [v for v in out.values() if v is not None])
+
+        sampling("top_k", 1, 3.0 * normal(20, 60000), top_k=40, top_p=0.9)
+        sampling("clusters", 3, 3.0 * normal(20, 60000), top_p=0.97)
+        sampling("value_runs", 2, (3.0 * normal(20, 60000)).bfloat16(), top_p=0.97)
+        rest = self.handles["rest"] = pkg.Sampler(max_rows=64, max_vocab=40000)
+        rest.set_overlap(overlap)
+        shard = normal(12, 40000)
+        candidates = rest.local_candidates(shard, 1000, 32)
+        merged = rest.merge_candidates(candidates.view(1, 12, 32), pkg.make_row_params(12, seed=6, top_k=32), 32)
+
+        def shards(stream):
+            rest.local_candidates(shard, 1000, 32, stream=stream, out=candidates)
+            rest.merge_candidates(candidates.view(1, 12, 32), None, 32, stream=stream, out=merged)
+        self.entries["shards"] = (2, shards, [candidates] + [v for v in merged.values() if v is not None])
+        for tokens, launches in ((32, 1), (400, 3)):
+            scores = normal(tokens, 96)
+            plan = rest.router_dispatch(scores, 4)
+            self.entries[f"router_{tokens}"] = (launches, lambda stream, scores=scores, plan=plan: rest.router_dispatch(scores, 4, stream=stream, out=plan),
+                                                [plan.expert_offsets, plan.route_token, plan.route_rank, plan.route_weight, plan.status])
+        hidden, ids = normal(64, 1536), torch.randint(64, (300,), generator=generator, device="cuda", dtype=torch.int32)
+        gathered = torch.empty((300, 1536), device="cuda")
+        library = pkg.library()
+
+        def gather(stream):
+            assert library.moe_regroup_gather(rest._handle, C.c_void_p(stream), C.c_void_p(hidden.data_ptr()), 64, 1536, C.c_void_p(ids.data_ptr()), 300,
+                                              C.c_void_p(gathered.data_ptr())) == 0
+        self.entries["gather"] = (1, gather, [gathered])
+        history = normal(6, 30000)
+        chosen = torch.empty((6, 512), dtype=torch.int32, device="cuda")
+
+        def index(stream):
+            assert library.moe_indexer_topk(rest._handle, C.c_void_p(stream), C.c_void_p(history.data_ptr()), 6, 30000, C.c_size_t(30000), 512,
+                                            C.c_void_p(chosen.data_ptr()), None) == 0
+        self.entries["indexer"] = (1, index, [chosen])
+        torch.cuda.synchronize()
+        self.torch = torch
+        for _, call, _ in self.entries.values():
+            call(torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        self.want = {name: [t.clone() for t in outputs] for name, (_, _, outputs) in self.entries.items()}
+        self.clear()
+
+    def clear(self):
+        for _, _, outputs in self.entries.values():
+            for t in outputs:
+                t.fill_(0)
+        self.torch.cuda.synchronize()
+
+    def compare(self):
+        self.torch.cuda.synchronize()
+        for name, (_, _, outputs) in self.entries.items():
+            for got, want in zip(outputs, self.want[name]):
+                assert self.torch.equal(got, want), name
+        self.clear()
+
+    def close(self):
+        for handle in self.handles.values():
+            handle.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("overlap", [False, True])
+def test_all_kernels_after_one_another_on_one_stream(pkg, torch_cuda, overlap):
+    """Every kernel of the library behind every other, three times over and nothing waited for in between, on the default stream
+    and on a stream of the caller's; the same with overlapping sampler launches (no input depends on an earlier call)."""
+    torch = torch_cuda
+    calls = Calls(pkg, torch, overlap)
+    try:
+        names = list(calls.entries)
+        streams = [torch.cuda.current_stream(), torch.cuda.Stream(), torch.cuda.Stream(priority=-1)]
+        for stream in streams:
+            for shift in range(len(names)):
+                for _ in range(3):
+                    for i in range(len(names)):
+                        calls.entries[names[(i * (shift + 1)) % len(names)]][1](stream.cuda_stream)
+                for name in names:
+                    calls.entries[name][1](stream.cuda_stream)
+                calls.compare()
+    finally:
+        calls.close()
+
+
+@pytest.mark.gpu
+def test_every_call_can_be_captured(pkg, torch_cuda):
+    """Each call with resident parameters becomes a graph of exactly its kernels, alone and all of them in one graph."""
+    torch = torch_cuda
+    calls = Calls(pkg, torch)
+    graphs = []
+    try:
+        for name, (launches, call, _) in calls.entries.items():
+            graphs.append(Captured(torch, call))
+            assert (graphs[-1].nodes, graphs[-1].kernels) == (launches, launches), name
+        for _ in range(2):
+            for graph in graphs:
+                graph.run()
+            calls.compare()
+        together = Captured(torch, lambda stream: [call(stream) for _, call, _ in calls.entries.values()])
+        graphs.append(together)
+        assert together.kernels == sum(launches for launches, _, _ in calls.entries.values())
+        for _ in range(2):
+            together.run()
+            calls.compare()
+    finally:
+        for graph in graphs:
+            graph.close()
+        calls.close()
