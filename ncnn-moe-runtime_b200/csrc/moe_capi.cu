@@ -1014,7 +1014,8 @@ int moe_indexer_topk(moe_sampler* sampler, void* stream_handle, const float* sco
     if (scores == nullptr || out_index == nullptr)
         return fail(sampler, MOE_STATUS_INVALID_ARGUMENT, "scores and out_index must not be null");
     DeviceGuard guard(sampler->device);
-    MOE_CUDA_CHECK(sampler, launch_indexer_topk(scores, rows, count, row_stride, top_k, out_index, out_score, static_cast<cudaStream_t>(stream_handle)));
+    MOE_CUDA_CHECK(sampler, launch_indexer_topk(scores, rows, count, row_stride, top_k, out_index, out_score, sampler->sm_count,
+                                                static_cast<cudaStream_t>(stream_handle)));
     return MOE_STATUS_OK;
 }
 

@@ -4,7 +4,8 @@
 // scored_index_precedes, :257-262 — score descending, index ascending on equal
 // scores — and the first index_top_k indices in that order).
 //
-// One CTA per row.  The row is read once: as much of it as fits stays in shared
+// Rows of up to 1024 scores are put in order whole, one record per thread (indexer_short_rows_kernel).
+// Longer ones: one CTA per row.  The row is read once: as much of it as fits stays in shared
 // memory (40 000 scores), later passes read the rest again from L2.  The 32-bit
 // order-preserving keys are counted by their upper 14 bits, which spreads
 // ordinary scores over a hundred counters and more (a byte digit leaves them in a
@@ -12,15 +13,18 @@
 // inside it are ranked against each other while they are few, and by two more
 // digits (14 and 4 bits) otherwise — equal scores, lowest indices first.  The
 // taken (key, index) records — the record and ordering primitive of the sampler —
-// are put in order by a monotone map of their keys onto 8192 buckets and a look
+// are put in order by a monotone map of their keys onto 4096 or 8192 buckets and a look
 // inside each bucket, or, where keys pile up, by a bitonic network that runs in
 // registers for strides inside a warp and through shared memory for the others.
 //
 // What bounds it: latency and shared-memory instructions of one SM per row.  With
 // byte digits, match.any aggregation, six passes over L2 and a bitonic sort in
 // shared memory, before and after: 64 rows x 40000 scores, top 2048 82.0 -> 27.3 us;
-// 128 x 131072, top 2048 263 -> 72; 64 x 2300, top 2048 30 -> 12; 128 x 1024, top 512
-// 14 -> 11.
+// 64 x 131072, top 2048 260 -> 72; 64 x 2300, top 2048 30.0 -> 11.4; 1000 x 2300, top
+// 512 75.7 -> 50.7; 64 x 1024, top 512 13.3 -> 6.6; 4000 x 300, top 64 130 -> 59.  What
+// got slower: rows between 1024 and some 9000 scores that nearly all agree in the upper
+// 14 key bits take all three digits and the network (1000 x 2300, top 512, 1 + 1e-6 N(0,1)
+// 76.8 -> 87.3; 64 of them 16.8 -> 16.6; top 64 12.7 -> 15.7).
 
 #include "moe_common.cuh"
 #include "moe_internal.h"
@@ -38,13 +42,16 @@ constexpr uint32_t kDigits = 1u << kDigitBits;
 constexpr uint32_t kResidentScores = (227u * 1024u - 5u * 1024u - kDigits * 4u) / 16u * 4u;
 constexpr uint32_t kZeroDigit = 0x80000000u >> (32 - kDigitBits); // zeros, the most common score by far
 constexpr uint32_t kCandidates = 512;   // entries of the boundary digit that are ranked directly
-constexpr uint32_t kOrderKeys = 8192;   // buckets of the final order
+// buckets of the final order; fewer of them where two CTAs share an SM
+template<int kCtas>
+constexpr uint32_t kOrderKeysFor = kCtas == 1 ? 8192u : 4096u;
 // Records a bucket may hold (else the bitonic network): a look inside costs n / 32 x records shared loads, and the
 // network for 1024 to 2048 records as much as about 4000 of them.
 __device__ __forceinline__ uint32_t order_limit(uint32_t n)
 {
     return min(256u, 131072u / max(n, 1u));
 }
+constexpr size_t kHalfSharedBytes = 113u * 1024u; // of an SM's 228 KiB, with 1 KiB per CTA for the system
 constexpr size_t kRowOffset = sizeof(uint32_t) * kDigits + 5u * 1024u; // of the resident scores in shared memory
 
 struct IndexerShared
@@ -117,13 +124,13 @@ __device__ __forceinline__ void count_digit(uint32_t* hist, uint32_t digit, bool
         atomicAdd(hist + digit, 1u);
 }
 
-// Descending order of kItems * kIndexThreads records, thread-major by warp: element j of a thread is
+// Descending order of kItems * kThreads records, thread-major by warp: element j of a thread is
 // position warp * 32 * kItems + 32 * j + lane.  `buffer` holds two images of the list.
-template<int kItems>
+template<int kItems, int kThreads>
 __device__ void bitonic_descending(uint64_t (&v)[kItems], uint64_t* buffer)
 {
     constexpr uint32_t kWarpSpan = 32u * kItems;
-    constexpr uint32_t kTotal = kIndexThreads * kItems;
+    constexpr uint32_t kTotal = kThreads * kItems;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t first = (threadIdx.x >> 5) * kWarpSpan + lane;
     uint32_t image = 0;
@@ -182,10 +189,44 @@ __device__ void bitonic_descending(uint64_t (&v)[kItems], uint64_t* buffer)
     }
 }
 
-template<int kItems>
-__global__ void __launch_bounds__(kIndexThreads) indexer_topk_kernel(const float* scores, uint32_t count, size_t row_stride, uint32_t top_k,
+// A short row (at most kThreads scores): the network puts all of it in rank order, one record per thread; the scores decide
+// nothing about the time.  What bounds it: shuffles and barriers.  The digits' counters cost the same whatever the row's
+// length and fill most of an SM: 4000 rows x 300, top 64 took 231 us, 130 with byte digits.
+template<int kThreads>
+__global__ void __launch_bounds__(kThreads) indexer_short_rows_kernel(const float* scores, uint32_t count, size_t row_stride, uint32_t top_k, uint32_t* out_index,
+                                                                      float* out_score)
+{
+    __shared__ uint64_t buffer[2 * kThreads];
+    const uint32_t tid = threadIdx.x;
+    wait_for_previous_kernel();
+    const float* row = scores + static_cast<size_t>(blockIdx.x) * row_stride;
+    const uint32_t selected = min(top_k, count);
+    out_index += static_cast<size_t>(blockIdx.x) * top_k;
+    if (out_score != nullptr)
+        out_score += static_cast<size_t>(blockIdx.x) * top_k;
+    uint64_t v[1] = {tid < count ? make_record(score_key(row[tid]), tid) : 0ull};
+    bitonic_descending<1, kThreads>(v, buffer);
+    if (tid < selected)
+    {
+        const uint32_t index = record_index(v[0]);
+        out_index[tid] = index;
+        if (out_score != nullptr)
+            out_score[tid] = row[index];
+    }
+    for (uint32_t position = selected + tid; position < top_k; position += kThreads)
+    {
+        out_index[position] = 0xFFFFFFFFu;
+        if (out_score != nullptr)
+            out_score[position] = 0.0f;
+    }
+}
+
+// kCtas: CTAs per SM.
+template<int kItems, int kCtas>
+__global__ void __launch_bounds__(kIndexThreads, kCtas) indexer_topk_kernel(const float* scores, uint32_t count, size_t row_stride, uint32_t top_k,
                                                                      uint32_t resident_fours, uint32_t* out_index, float* out_score)
 {
+    constexpr uint32_t kOrderKeys = kOrderKeysFor<kCtas>;
     extern __shared__ __align__(16) unsigned char shared_raw[];
     uint32_t* const hist = reinterpret_cast<uint32_t*>(shared_raw);
     IndexerShared& sh = *reinterpret_cast<IndexerShared*>(shared_raw + sizeof(uint32_t) * kDigits);
@@ -553,45 +594,79 @@ __global__ void __launch_bounds__(kIndexThreads) indexer_topk_kernel(const float
     for (int j = 0; j < kItems; ++j)
         v[j] = records[first + 32u * j];
     __syncthreads();
-    bitonic_descending<kItems>(v, reinterpret_cast<uint64_t*>(shared_raw + kRowOffset));
+    bitonic_descending<kItems, kIndexThreads>(v, reinterpret_cast<uint64_t*>(shared_raw + kRowOffset));
 #pragma unroll
     for (int j = 0; j < kItems; ++j)
         if (first + 32u * j < above_total)
             write(first + 32u * j, v[j]);
 }
 
-template<int kItems>
-cudaError_t launch_indexer(const float* scores, uint32_t rows, uint32_t count, size_t row_stride, uint32_t top_k, uint32_t* out_index, float* out_score,
-                           cudaStream_t stream)
+// groups of four scores kept in shared memory
+uint32_t resident_fours_of(uint32_t count)
+{
+    const uint32_t fours = count / 4u + (count % 4u != 0u ? 1u : 0u);
+    return fours < kResidentScores / 4u ? fours : kResidentScores / 4u;
+}
+template<int kItems, int kCtas>
+size_t indexer_shared_bytes(uint32_t count)
 {
     // the buckets and the ordered records, or the network's two images of the list, take the place of the resident scores
     const size_t list_bytes = sizeof(uint64_t) * kItems * kIndexThreads;
-    const size_t sort_bytes = list_bytes + (list_bytes > sizeof(uint32_t) * kOrderKeys ? list_bytes : sizeof(uint32_t) * kOrderKeys);
-    const uint32_t resident_fours = (count + 3u) / 4u < kResidentScores / 4u ? (count + 3u) / 4u : kResidentScores / 4u;
-    const size_t row_bytes = sizeof(float) * 4u * resident_fours;
-    const size_t shared_bytes = kRowOffset + (row_bytes > sort_bytes ? row_bytes : sort_bytes);
+    const size_t bucket_bytes = sizeof(uint32_t) * kOrderKeysFor<kCtas>;
+    const size_t sort_bytes = list_bytes + (list_bytes > bucket_bytes ? list_bytes : bucket_bytes);
+    const size_t row_bytes = sizeof(float) * 4u * resident_fours_of(count);
+    return kRowOffset + (row_bytes > sort_bytes ? row_bytes : sort_bytes);
+}
+
+template<int kItems, int kCtas>
+cudaError_t launch_indexer(const float* scores, uint32_t rows, uint32_t count, size_t row_stride, uint32_t top_k, uint32_t* out_index, float* out_score,
+                           int sm_count, cudaStream_t stream)
+{
+    if constexpr (kCtas == 1 && kItems <= 2)
+    {
+        // More rows than SMs: two CTAs share one, if their rows and lists fit.  A CTA alone is a little faster with all the
+        // registers and buckets (64 x 40000, top 2048: 27.3 us, 29.1 without), but waits a good part of its time: 1000 rows x
+        // 2300, top 512 62.7 -> 50.7 us, 1000 x 9000, top 2048 91.5 -> 79.4.
+        if (rows > static_cast<uint32_t>(sm_count) && indexer_shared_bytes<kItems, 2>(count) <= kHalfSharedBytes)
+            return launch_indexer<kItems, 2>(scores, rows, count, row_stride, top_k, out_index, out_score, sm_count, stream);
+    }
+    const size_t shared_bytes = indexer_shared_bytes<kItems, kCtas>(count);
     static SharedOptIn opt_in;
-    if (cudaError_t status = opt_in_shared(opt_in, indexer_topk_kernel<kItems>, shared_bytes))
+    if (cudaError_t status = opt_in_shared(opt_in, indexer_topk_kernel<kItems, kCtas>, shared_bytes))
         return status;
-    return launch_following(indexer_topk_kernel<kItems>, rows, kIndexThreads, shared_bytes, stream, scores, count, row_stride, top_k, resident_fours, out_index,
-                            out_score);
+    return launch_following(indexer_topk_kernel<kItems, kCtas>, rows, kIndexThreads, shared_bytes, stream, scores, count, row_stride, top_k,
+                            resident_fours_of(count), out_index, out_score);
+}
+
+template<int kThreads>
+cudaError_t launch_short_rows(const float* scores, uint32_t rows, uint32_t count, size_t row_stride, uint32_t top_k, uint32_t* out_index, float* out_score,
+                              cudaStream_t stream)
+{
+    if constexpr (kThreads < kIndexThreads)
+    {
+        if (count > kThreads)
+            return launch_short_rows<2 * kThreads>(scores, rows, count, row_stride, top_k, out_index, out_score, stream);
+    }
+    return launch_following(indexer_short_rows_kernel<kThreads>, rows, kThreads, 0, stream, scores, count, row_stride, top_k, out_index, out_score);
 }
 
 } // namespace
 
 cudaError_t launch_indexer_topk(const float* scores, uint32_t rows, uint32_t count, size_t row_stride, uint32_t top_k, uint32_t* out_index,
-                                float* out_score, cudaStream_t stream)
+                                float* out_score, int sm_count, cudaStream_t stream)
 {
     if (rows == 0 || top_k == 0)
         return cudaSuccess;
+    if (count <= kIndexThreads) // one record per thread
+        return launch_short_rows<32>(scores, rows, count, row_stride, top_k, out_index, out_score, stream);
     const uint32_t selected = top_k < count ? top_k : count;
     if (selected <= kIndexThreads)
-        return launch_indexer<1>(scores, rows, count, row_stride, top_k, out_index, out_score, stream);
+        return launch_indexer<1, 1>(scores, rows, count, row_stride, top_k, out_index, out_score, sm_count, stream);
     if (selected <= 2u * kIndexThreads)
-        return launch_indexer<2>(scores, rows, count, row_stride, top_k, out_index, out_score, stream);
+        return launch_indexer<2, 1>(scores, rows, count, row_stride, top_k, out_index, out_score, sm_count, stream);
     if (selected <= 4u * kIndexThreads)
-        return launch_indexer<4>(scores, rows, count, row_stride, top_k, out_index, out_score, stream);
-    return launch_indexer<8>(scores, rows, count, row_stride, top_k, out_index, out_score, stream);
+        return launch_indexer<4, 1>(scores, rows, count, row_stride, top_k, out_index, out_score, sm_count, stream);
+    return launch_indexer<8, 1>(scores, rows, count, row_stride, top_k, out_index, out_score, sm_count, stream);
 }
 
 } // namespace moe

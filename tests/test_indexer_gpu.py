@@ -76,3 +76,32 @@ def test_boundaries_of_the_selection(sampler, checker, torch_cuda, count, top_k)
     rows[8, rng.choice(count, 40, replace=False)] = np.inf
     rows[8, rng.choice(count, 40, replace=False)] = -np.inf
     check(sampler, checker, torch_cuda, rows, top_k, count=count)
+
+
+@pytest.mark.parametrize("count", [1, 2, 31, 32, 33, 63, 64, 65, 127, 129, 255, 257, 511, 513, 1023, 1024])
+@pytest.mark.parametrize("top_k", [1, 32, 100, 1024, 2000])
+def test_short_rows(sampler, checker, torch_cuda, count, top_k):
+    """Rows of one record per thread, around every number of threads: all of the row is put in order."""
+    rng = np.random.default_rng(count)
+    rows = np.empty((6, count + 1), dtype=np.float32)
+    normal = rng.standard_normal((6, count + 1)).astype(np.float32)
+    rows[0] = normal[0]
+    rows[1] = np.maximum(normal[1], 0.0)
+    rows[2] = np.round(normal[2] * 2.0) / 2.0
+    rows[3] = np.where(normal[3] > 0.0, normal[3] * 1e-41, -0.0)
+    rows[4] = 7.25
+    rows[5] = normal[5]
+    rows[5, rng.integers(count)] = np.inf
+    rows[5, rng.integers(count)] = -np.inf
+    check(sampler, checker, torch_cuda, rows, top_k, count=count)
+
+
+@pytest.mark.parametrize("count,top_k", [(1025, 64), (2049, 1024), (2300, 2048), (9001, 2048), (11264, 512), (11265, 512), (11264, 2048), (3000, 3000)])
+def test_more_rows_than_sms(sampler, checker, torch_cuda, count, top_k):
+    """Two CTAs share an SM while the row and the lists of both fit (11264 scores), one takes it otherwise."""
+    rng = np.random.default_rng(count)
+    rows = rng.standard_normal((320, count)).astype(np.float32)
+    rows[1::4] = np.maximum(rows[1::4], 0.0)
+    rows[2::4] = np.round(rows[2::4] * 4.0) / 4.0
+    rows[3::4] = 1.0 + 1e-6 * rows[3::4]
+    check(sampler, checker, torch_cuda, rows, top_k)
