@@ -234,6 +234,12 @@ __device__ __forceinline__ void wait_for_previous_kernel()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Lets the next kernel of the stream begin (up to its wait) once every CTA of this one has called it or exited.
+__device__ __forceinline__ void grid_dependency_release()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- warp / block reductions ------------------------------------------------------
 __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v)
 {

@@ -1263,8 +1263,11 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
         }
     }
 }
+    grid_dependency_release(); // every cluster is resident: the one-CTA kernel behind takes no place from any
 
 // CTAs per row.  A row costs a part that does not shrink with the cluster (barriers, scans, sequential
+    if (pending == 0)
+        return; // the counters are as the next call needs them
 // adds: about 45 us) and a part that does (the passes over its items: about 200 us at 150000 logits);
 // clusters run side by side as far as the device holds them.  The size with the smallest
 // rounds x (fixed + passes / size) wins.  Measured with clusters of 1, 2, 4, 8, 16 CTAs, us per call:

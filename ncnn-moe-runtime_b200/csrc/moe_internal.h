@@ -106,6 +106,8 @@ struct SampleArgs
     // while the previous kernel of the stream is still finishing, so it waits
     // for that kernel (griddepcontrol.wait) before its first global write
     bool overlap_previous;
+    // the exact kernels follow in the same call and may take their places on the SMs while this one runs
+    bool release_exact;
 };
 
 cudaError_t launch_sample_rows(const SampleArgs& args, const Workspace& ws, uint32_t splits, cudaStream_t stream);

@@ -1418,6 +1418,8 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_kernel(const Sa
     uint32_t* const count = kDeferred ? ws.exact_deferred_count : ws.exact_count;
     const uint32_t* const entries = kDeferred ? ws.exact_deferred : ws.exact_rows;
     const uint32_t pending = *count;
+    if (kDeferred && pending == 0)
+        return; // the counters are as the next call needs them (an early exit costs the other variants registers)
     const uint32_t slot_stride = (ws.max_vocab + 3u) & ~3u;
     uint32_t* slot_keys = ws.sort_keys + static_cast<size_t>(blockIdx.x) * 4u * slot_stride;
     // rows cost from a few to several hundred microseconds: a CTA takes the next one when it is free

@@ -110,14 +110,6 @@ namespace moe {
 
 namespace {
 
-// Programmatic dependent launch (sm_90+).  `wait` blocks until every kernel this
-// launch depends on has completed and its memory is visible; `launch_dependents`
-// lets the next kernel of the stream begin once all CTAs have issued it or exited.
-__device__ __forceinline__ void grid_dependency_release()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 #ifndef MOE_ROW_MIN_CTAS
 #define MOE_ROW_MIN_CTAS 2 // CTAs per SM the register allocation leaves room for
 #endif
@@ -1472,7 +1464,11 @@ __global__ void __launch_bounds__(kThreads, MOE_ROW_MIN_CTAS) sample_rows_kernel
     if (a.overlap_previous)
         grid_dependency_release();
     else
+    {
         wait_for_previous_kernel();
+        if (a.release_exact)
+            grid_dependency_release(); // the exact kernels are on the SMs, waiting, when this one ends
+    }
 
     // ---- the slice of this CTA, and its first bytes on request at once -----------
     const T* row_pointer = row_logits<T>(a, row);

@@ -282,3 +282,38 @@ def test_every_call_can_be_captured(pkg, torch_cuda):
         for graph in graphs:
             graph.close()
         calls.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 16, 64, 65, 200])
+@pytest.mark.parametrize("overlap", [False, True])
+def test_calls_with_and_without_rows_for_the_exact_kernels(pkg, torch_cuda, rows, overlap):
+    """Batches that finish on chip, batches that do not and batches some of whose rows the clusters leave, one after the other
+    and nothing waited for: the exact kernels of each find the list of their own call."""
+    torch = torch_cuda
+    vocab = 30011
+    generator = torch.Generator(device="cuda").manual_seed(rows)
+    peaked = 12.0 * torch.randn((rows, vocab), generator=generator, device="cuda")
+    alive = 2.0 * torch.randn((rows, vocab), generator=generator, device="cuda")
+    mixed = torch.where(torch.arange(rows, device="cuda")[:, None] % 3 == 0, peaked, alive)
+    mixed[1::3] = mixed[1::3].bfloat16().float()          # left to the one-CTA kernel
+    sampler = pkg.Sampler(max_rows=rows, max_vocab=vocab)
+    try:
+        params = pkg.make_row_params(rows, seed=4, temperature=0.8, top_p=0.97)
+        kinds = (peaked, alive, mixed)
+        want = []
+        for logits in kinds:
+            want.append(sampler.sample_batch(logits, params))
+            torch.cuda.synchronize()
+        sampler.set_overlap(overlap)
+        order = [0, 0, 1, 0, 2, 2, 1, 1, 0, 2, 0, 1, 2, 0]
+        got = [{k: torch.empty_like(v) if v is not None else None for k, v in want[0].items()} for _ in order]
+        torch.cuda.synchronize()
+        for kind, out in zip(order, got):
+            sampler.sample_batch(kinds[kind], None, out=out)
+        torch.cuda.synchronize()
+        for kind, out in zip(order, got):
+            for name in ("token", "probability", "flags", "status"):
+                assert torch.equal(out[name], want[kind][name]), (kind, name)
+    finally:
+        sampler.close()
