@@ -22,10 +22,10 @@
 //     the live window, a check that fails) is listed for the one-CTA kernel that runs behind this one.
 //
 // What bounds it: for one to twenty rows latency (about twenty cluster barriers and block scans, the
-// sequential adds of the head); for hundreds of rows the issue slots of the item passes (about 230 warp
-// instructions per 32 logits, 49 % of the issue slots with one CTA per row).  The one-CTA path it replaces
-// for these rows put all live items in rank order first.  Per call of 151936 logits a row, Top-P only:
-// 1 row 568 -> 145 us, 8 rows 594 -> 160, 64 rows 680 -> 304, 256 rows 1806 -> 880.
+// sequential adds of the head); for hundreds of rows the issue slots of the item passes.  The one-CTA path
+// it replaces for these rows put all live items in rank order first.  Calls of rows of 151936 logits
+// 3 N(0,1), T 0.9, Top-P 0.95, streaming kernel included: 1 row 433 -> 123 us, 8 rows 450 -> 139, 64 rows
+// 517 -> 313, 256 rows 1378 -> 734.
 
 #include <cooperative_groups.h>
 
@@ -55,17 +55,25 @@ namespace cg = cooperative_groups;
 #endif
 
 constexpr uint32_t kGroups = 16384;
-constexpr uint32_t kGroupLimit = 120;    // items per group: 120 steps of at most 2^24 fit 32 bits
+// Items per group: as many as the literal list takes (equal logits, such as those of a padded vocabulary, share a group).
+// An item behind the head is at most 1/kHead of the accumulator, which is below 2^24 units: its step is below kStepLimit
+// unless the unit was guessed far too small, and kGroupLimit such steps fit the 31 bits of a counter.  The limit ends in
+// one half, so that an item that reaches it looks like a tie and makes its group literal.
+// With 120 items per group rows with 267 equal logits were left after two passes: 8 of them took 629 us, 604 without
+// the clusters, 138 now; 256 of them 2690, 2280 and 765.
+constexpr uint32_t kGroupLimit = 3072;
+constexpr float kStepLimit = 131071.5f;
 constexpr uint32_t kHead = 192;          // candidates added literally, rounded up to whole groups
-constexpr uint32_t kHeadCapacity = 512;  // >= kHead + kGroupLimit
+constexpr uint32_t kHeadCapacity = 512;
 constexpr uint32_t kLiteralGroups = 96;
-constexpr uint32_t kLiteralItems = 2048;
+constexpr uint32_t kLiteralItems = 3072; // dense rows (90 items a group) mark up to thirty groups that refining does not spare
 constexpr uint32_t kMaxCluster = 16;
 constexpr uint32_t kDeadGroup = 0xFFFFu;
 constexpr int kGuardUnits = 64;          // a group this close to the end of a binade or to the bound is literal
 constexpr int kMaxGuesses = 5;
 constexpr uint32_t kTieBit = 0x80000000u; // of a group's step counter: some item is a tie
-static_assert(kHead + kGroupLimit <= kHeadCapacity, "the head holds whole groups");
+static_assert(kGroupLimit <= kLiteralItems, "a group that has to be added literally fits the list");
+static_assert((1u << 24) / kHead < 131071u && static_cast<uint64_t>(kGroupLimit) * 131072u < kTieBit, "the steps of a group fit its counter");
 
 struct LiteralGroup
 {
@@ -111,18 +119,20 @@ struct ClusterStats
 struct alignas(16) ClusterShared
 {
     uint32_t table[kGroups];   // per group: count, then steps of the current sum
-    uint8_t count[kGroups];    // items of the group over the whole cluster
+    uint16_t count[kGroups];   // items of the group over the whole cluster
     uint8_t exponent[kGroups]; // guessed exponent of the accumulator before the group, biased by 127
     uint32_t literal_bits[kGroups / 32];
     // rank 0 only
     uint64_t head_in[kHeadCapacity];
     uint64_t head[kHeadCapacity];
     float head_value[kHeadCapacity];
-    uint64_t item_in[kLiteralItems];
-    uint64_t item[kLiteralItems];
+    uint64_t item[kLiteralItems];          // as they come, and in rank order
+    uint64_t item_by_group[kLiteralItems]; // in between: group by group
     float item_value[kLiteralItems];
     LiteralGroup literal_in[kLiteralGroups];
     LiteralGroup literal[kLiteralGroups];
+    uint32_t literal_begin[kLiteralGroups]; // where the group's items stand in the list
+    uint32_t literal_end[kLiteralGroups];
     uint32_t head_count, item_count, literal_count;
     uint32_t literal_items; // items of the literal groups
     // every CTA
@@ -132,6 +142,7 @@ struct alignas(16) ClusterShared
     float warp_sum[kExactWarps];
     uint32_t overfull;
     uint32_t head_end;
+    uint32_t head_total; // candidates of the head
     uint32_t entry;
     Jump jump[kMaxGuesses];
     SumState state;
@@ -327,17 +338,17 @@ __device__ __noinline__ void guess_exponents(ClusterShared& cs, uint32_t first_g
 {
     static_assert(kGroups == 16u * kExactThreads, "a thread guesses for sixteen groups");
     const uint32_t tid = threadIdx.x;
-    const uint4 packed = *reinterpret_cast<const uint4*>(cs.count + 16u * tid);
-    uint32_t word[4] = {packed.x, packed.y, packed.z, packed.w};
+    const uint2* const words = reinterpret_cast<const uint2*>(cs.count + 16u * tid);
     float items[4], addend[4];
     int exponent[4] = {0, 0, 0, 0};
 #pragma unroll
     for (uint32_t k = 0; k < 4u; ++k)
     {
         const uint32_t g = 16u * tid + 4u * k;
-        if (g < first_group)
-            word[k] = g + 4u <= first_group ? 0u : word[k] >> (8u * (first_group - g));
-        items[k] = static_cast<float>(__dp4a(word[k], 0x01010101u, 0u));
+        const uint2 four = words[k];
+        const uint32_t n = (g >= first_group ? four.x & 0xFFFFu : 0u) + (g + 1u >= first_group ? four.x >> 16 : 0u)
+                           + (g + 2u >= first_group ? four.y & 0xFFFFu : 0u) + (g + 3u >= first_group ? four.y >> 16 : 0u);
+        items[k] = static_cast<float>(n);
         addend[k] = factor * exp2f(-static_cast<float>(g + 2u) * log2_step);
     }
 #pragma unroll
@@ -496,7 +507,7 @@ __device__ __forceinline__ void add_steps(const StepArgs& s, ClusterShared& cs, 
                 value = divide_by(value, s.kept_total, s.kept_reciprocal);
             uint32_t exponent;
             asm("ld.shared.u8 %0, [%1];" : "=r"(exponent) : "r"(exponent_base + (active[u] ? g[u] : 0u)));
-            t[u] = fminf(value * __uint_as_float((277u - exponent) << 23), 16777216.0f); // value / unit
+            t[u] = fminf(value * __uint_as_float((277u - exponent) << 23), kStepLimit); // value / unit
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
@@ -625,6 +636,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
         cs.item_count = 0;
         cs.literal_count = 0;
         cs.head_end = kGroups;
+        cs.head_total = 0;
         cs.stats[rank] = ClusterStats{0u, 0xFFFFFFFFu, 0u, 0u, 0u};
     }
     __syncthreads();
@@ -736,16 +748,20 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
         {
             const uint32_t n = cs.table[owned_begin + i];
             over |= n > kGroupLimit;
-            cs.count[owned_begin + i] = static_cast<uint8_t>(min(n, 255u));
+            cs.count[owned_begin + i] = static_cast<uint16_t>(min(n, 65535u));
         }
         __syncthreads();
-        // my counts to every peer, sixteen bytes per thread
-        const uint32_t packs = owned / 16u;
-        static_assert(kGroups / 16u == kExactThreads, "one store per thread");
-        const uint32_t peer = tid / packs;
-        if (peer != rank)
-            reinterpret_cast<uint4*>(cluster.map_shared_rank(cs.count, peer) + owned_begin)[tid % packs] =
-                reinterpret_cast<const uint4*>(cs.count + owned_begin)[tid % packs];
+        // my counts to every peer, two stores of sixteen bytes per thread
+        const uint32_t packs = owned / 8u;
+        static_assert(kGroups / 8u == 2u * kExactThreads, "two stores per thread");
+#pragma unroll
+        for (uint32_t i = tid; i < kGroups / 8u; i += kExactThreads)
+        {
+            const uint32_t peer = i / packs;
+            if (peer != rank)
+                reinterpret_cast<uint4*>(cluster.map_shared_rank(cs.count, peer) + owned_begin)[i % packs] =
+                    reinterpret_cast<const uint4*>(cs.count + owned_begin)[i % packs];
+        }
         if (__any_sync(kFullMask, over) && lane < cluster_size)
             *cluster.map_shared_rank(&cs.overfull, lane) = 1u;
     }
@@ -757,9 +773,13 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
     uint32_t live_total;
     {
         constexpr uint32_t kPerThread = kGroups / kExactThreads;
-        const uint4 packed = *reinterpret_cast<const uint4*>(cs.count + tid * kPerThread);
-        const uint32_t sum = __dp4a(packed.x, 0x01010101u, 0u) + __dp4a(packed.y, 0x01010101u, 0u) + __dp4a(packed.z, 0x01010101u, 0u)
-                             + __dp4a(packed.w, 0x01010101u, 0u);
+        uint32_t sum = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kPerThread / 2u; ++j)
+        {
+            const uint32_t two = reinterpret_cast<const uint32_t*>(cs.count + tid * kPerThread)[j];
+            sum += (two & 0xFFFFu) + (two >> 16);
+        }
         uint64_t total;
         const uint32_t inclusive = static_cast<uint32_t>(block_scan_u64(sum, cs.warp_total, total));
         uint32_t before = inclusive - sum;
@@ -771,6 +791,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                 if (before >= kHead)
                 {
                     cs.head_end = tid * kPerThread + j + 1u;
+                    cs.head_total = before;
                     break;
                 }
             }
@@ -780,6 +801,8 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
     }
     CL_MARK(18);
     const uint32_t head_end = cs.head_end; // groups below it are the head
+    if (cs.head_total > kHeadCapacity)
+        return false; // its last group piles up
     const bool all_listed = live_total == finite_total;
 
     // groups behind this one hold nobody that passes the Min-P floor (the slack covers every rounding)
@@ -806,6 +829,13 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
             active_last = min(last_group, group_of(key_to_float(record_key(threshold))));
         const float factor = sum == 0 ? 1.0f : (sum == 1 ? 1.0f / total : 1.0f / total / kept_total);
         guess_exponents(cs, sum == 0 ? 0u : head_end, sum == 0 ? 0.0f : head_acc, factor, log2_step);
+        if (sum == 0 && head_end < 4u)
+        {
+            // nothing stands before the first four groups, but the head may end among them: its addends are close to one
+            if (tid < 4u)
+                cs.exponent[tid] = static_cast<uint8_t>(exponent_of(static_cast<float>(cs.head_total) * exp2f(-2.0f * log2_step)) + 127);
+            __syncthreads();
+        }
         CL_MARK(19);
         // the fixed-point unit: one binade below the first guess while the head's sum is not known yet
         const int base_exponent = sum == 0 ? (head_end < kGroups ? static_cast<int>(cs.exponent[head_end]) - 128 : -1) : exponent_of(head_acc);
@@ -951,7 +981,10 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
             };
             if (literal_groups > kLiteralGroups || literal_items > kLiteralItems)
             {
-                // the guess was too far off: repeat with the exponents of the accumulators just found
+                // the guess was too far off: repeat with the exponents of the accumulators just found; a better guess that
+                // marks few groups with too many items shows that refining does not help
+                if (guess > 0 && literal_groups <= kLiteralGroups)
+                    return false;
                 publish_exponents(0u);
                 jump_count = 0;
                 if (tid == 0)
@@ -987,7 +1020,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                         hits &= hits - 1u;
                         const uint32_t slot = atomicAdd(&first_cta.item_count, 1u);
                         if (slot < kLiteralItems)
-                            first_cta.item_in[slot] = make_record(ordered_key(row_pointer[i]), i);
+                            first_cta.item[slot] = make_record(ordered_key(row_pointer[i]), i);
                     }
                 }
             }
@@ -1007,14 +1040,51 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                 }
                 else
                 {
-                    rank_records(cs.item_in, cs.item, items);
-                    // the literal groups in rank order
+                    // the literal groups in rank order, and where the items of each stand
                     if (tid < literal_groups)
                     {
-                        uint32_t before = 0;
+                        uint32_t before = 0, items_before = 0;
                         for (uint32_t j = 0; j < literal_groups; ++j)
-                            before += cs.literal_in[j].group < cs.literal_in[tid].group ? 1u : 0u;
+                        {
+                            const bool earlier = cs.literal_in[j].group < cs.literal_in[tid].group;
+                            before += earlier ? 1u : 0u;
+                            items_before += earlier ? cs.count[cs.literal_in[j].group] : 0u;
+                        }
                         cs.literal[before] = cs.literal_in[tid];
+                        cs.literal_begin[before] = items_before;
+                        cs.literal_end[before] = items_before; // grows to the end as the items come in
+                    }
+                    __syncthreads();
+                    // place in `literal` of an item's group
+                    const auto literal_of = [&](uint64_t record) {
+                        const uint32_t g = group_of(key_to_float(record_key(record)));
+                        uint32_t low = 0, high = literal_groups;
+                        while (high - low > 1u)
+                        {
+                            const uint32_t middle = (low + high) / 2u;
+                            if (cs.literal[middle].group <= g)
+                                low = middle;
+                            else
+                                high = middle;
+                        }
+                        return low;
+                    };
+                    for (uint32_t i = tid; i < items; i += kExactThreads)
+                    {
+                        const uint64_t record = cs.item[i];
+                        cs.item_by_group[atomicAdd(&cs.literal_end[literal_of(record)], 1u)] = record;
+                    }
+                    __syncthreads();
+                    // a group's items by their rank among themselves: comparing every two items of a dense row's 2400 took 180 us
+                    for (uint32_t i = tid; i < items; i += kExactThreads)
+                    {
+                        const uint64_t record = cs.item_by_group[i];
+                        const uint32_t at = literal_of(record);
+                        uint32_t rank_in_group = 0;
+#pragma unroll 4
+                        for (uint32_t j = cs.literal_begin[at]; j < cs.literal_end[at]; ++j)
+                            rank_in_group += cs.item_by_group[j] > record ? 1u : 0u;
+                        cs.item[cs.literal_begin[at] + rank_in_group] = record;
                     }
                     __syncthreads();
                     for (uint32_t i = tid; i < items; i += kExactThreads)
@@ -1193,8 +1263,11 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
     const uint32_t rank = cluster.block_rank();
     const uint32_t cluster_size = cluster.num_blocks();
     const uint32_t tid = threadIdx.x;
+    grid_dependency_release(); // every cluster is resident: the one-CTA kernel behind takes no place from any
     wait_for_previous_kernel();
     const uint32_t pending = *ws.exact_count;
+    if (pending == 0)
+        return; // the counters are as the next call needs them
     const uint32_t slot_stride = (ws.max_vocab + 3u) & ~3u;
     // the cluster's items (numerators, then group numbers) in the slot of its number, every CTA its slice
     const uint32_t cluster_index = blockIdx.x / cluster_size;
@@ -1263,16 +1336,15 @@ __global__ void __launch_bounds__(kExactThreads, 1) sample_exact_cluster_kernel(
         }
     }
 }
-    grid_dependency_release(); // every cluster is resident: the one-CTA kernel behind takes no place from any
 
-// CTAs per row.  A row costs a part that does not shrink with the cluster (barriers, scans, sequential
-    if (pending == 0)
-        return; // the counters are as the next call needs them
-// adds: about 45 us) and a part that does (the passes over its items: about 200 us at 150000 logits);
-// clusters run side by side as far as the device holds them.  The size with the smallest
-// rounds x (fixed + passes / size) wins.  Measured with clusters of 1, 2, 4, 8, 16 CTAs, us per call:
-// 1 row 253, 175, 137, 118, 112; 20 rows 355, 243, 190, 232, 324; 64 rows 420, 315, 378, 507, 855;
-// 256 rows 707, 750, 1032, 1680, 3193.
+// CTAs per row.  A row costs a part that does not shrink with the cluster (barriers, scans, sequential adds) and a
+// part that does (the passes over its items); clusters run side by side as far as the device holds them.  The size with the
+// smallest rounds x (fixed + passes / size) wins.  Alone, a call of one row fits 110 + 214 / size us; the 45 and 200 below
+// count a further round as what it adds while others run, and they choose the best measured size at every batch but one
+// (80 rows: 400 against 376).  Clusters of 1, 2, 4, 8, 16 CTAs, us per call, 151936 logits a row:
+// 1 row 324, 211, 161, 132, 124; 8 rows 331, 219, 167, 138, 182; 20 rows 333, 224, 170, 218, 313; 64 rows 352, 244, 317, 493,
+// 878; 100 rows 376, 397, 473, 719, 1315; 160 rows 605, 556, 692, 1119, 2101; 256 rows 736, 793, 1072, 1778, 3378.
+// The rows counted are those without Top-K; how many of them the streaming kernel hands over is not known here.
 cudaError_t launch_sample_exact_cluster(const SampleArgs& args, const Workspace& ws, uint32_t untruncated_rows, cudaStream_t stream)
 {
     static SharedOptIn opt_in;

@@ -83,6 +83,19 @@ def test_sums_that_are_repeated(pkg, parity, torch_cuda, size):
     assert counts["repeats"] > 0 and counts["refinements"] > 0
 
 
+@pytest.mark.parametrize("size", [1, 2, 4, 8, 16])
+def test_rows_that_are_dense_at_the_top(pkg, parity, torch_cuda, size):
+    """The head fills within the first four groups, before which there is no accumulator to guess an exponent from."""
+    rng = np.random.default_rng(12)
+    vocab = 120000
+    logits = np.stack([-rng.exponential(scale, vocab) for scale in (1.5, 2.0, 3.0, 4.0)]).astype(np.float32)
+    with Clusters(pkg, torch_cuda, parity.sampler, size) as clusters:
+        for top_p in (0.9, 0.999):
+            parity.check(logits, pkg.make_row_params(4, seed=size, top_k=0, top_p=top_p))
+        counts = clusters.counts()
+    assert counts["rows"] == 8 and counts["left"] == 0
+
+
 @pytest.mark.parametrize("size", [1, 4, 16])
 def test_rows_that_are_left(pkg, parity, torch_cuda, size):
     """Rows of bf16 values, rows with more equal logits than a group holds, and rows with a Top-K above the streaming limit
@@ -92,13 +105,37 @@ def test_rows_that_are_left(pkg, parity, torch_cuda, size):
     normal = (3.0 * rng.standard_normal((4, vocab))).astype(np.float32)
     widened = ((normal[1].view(np.uint32) >> 16) << 16).view(np.float32)
     filled = normal[2].copy()
-    filled[-300:] = np.float32(0.1)
+    filled[-4000:] = np.float32(0.1)
     logits = np.stack([normal[0], widened, filled, normal[3]])
     params = pkg.make_row_params(4, seed=1, top_k=np.array([0, 0, 0, 1500], dtype=np.uint32), temperature=1.5, top_p=0.99)
     with Clusters(pkg, torch_cuda, parity.sampler, size) as clusters:
         parity.check(logits, params)
         counts = clusters.counts()
     assert counts["rows"] == 1 and counts["left"] == 3
+
+
+@pytest.mark.parametrize("size", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("equal,most_left", [(119, 0), (121, 0), (255, 0), (257, 0), (1000, 5), (3000, 10), (3073, 20), (40000, 20)])
+def test_equal_logits_share_a_group(pkg, parity, torch_cuda, size, equal, most_left):
+    """Equal logits, as the padding of a vocabulary has them, wherever they lie: deep in the tail, where the bound or the draw may
+    fall among them, and in the head.  A group takes as many as the list of literal items, the head 512 candidates."""
+    rng = np.random.default_rng(equal)
+    vocab = 50021
+    rows = []
+    for value in (-12.0, -6.0, 0.0, 3.0, 9.0):
+        row = (3.0 * rng.standard_normal(vocab)).astype(np.float32)
+        row[rng.choice(vocab, equal, replace=False)] = np.float32(value + 1.0 / 1024.0)
+        rows.append(row)
+    logits = np.stack(rows)
+    with Clusters(pkg, torch_cuda, parity.sampler, size) as clusters:
+        for top_p in (0.6, 0.9, 0.999, 1.0):
+            params = pkg.make_row_params(len(rows), seed=equal + size, top_k=0, temperature=1.5, top_p=top_p, step=int(1000 * top_p))
+            parity.check(logits, params)
+        counts = clusters.counts()
+    assert counts["rows"] + counts["left"] == 4 * len(rows)
+    assert counts["left"] <= most_left
+    if equal > 3072:
+        assert counts["rows"] == 0
 
 
 @pytest.mark.parametrize("size", [1, 2, 16])
