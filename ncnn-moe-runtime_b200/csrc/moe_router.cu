@@ -156,6 +156,9 @@ __device__ __forceinline__ void warp_radix_select(uint64_t* records, uint32_t n,
 
 // Scores one token, selects its experts and their weights (out_expert, out_weight: top_k entries of this token) and
 // counts them in block_counts.  One warp; scores and records hold expert_count entries, radix_bins 256 (wide routers only).
+// kCached: a lane only looks for its best record again after it lost it.  That spares shared-memory traffic where sixteen warps
+// share an SM (32 tokens x 160 experts, top 8 8.9 against 9.3 us) and gains nothing in the kernel over all SMs.
+template<bool kCached>
 __device__ __forceinline__ void select_token(const RouterArgs& a, uint32_t token, float* scores, uint64_t* records, uint32_t* radix_bins,
                                              uint32_t* block_counts, unsigned long long* error_word, uint32_t* out_expert, float* out_weight)
 {
@@ -256,16 +259,14 @@ __device__ __forceinline__ void select_token(const RouterArgs& a, uint32_t token
             warp_radix_select(records, experts, top_k, radix_bins);
             pool = top_k;
         }
-        // every lane keeps the best of its records; only the lane that owned a winner looks again
         uint64_t best = 0ull;
         uint32_t best_slot = 0;
         bool look = true;
         for (uint32_t r = 0; r < top_k; ++r)
         {
-            if (look)
+            if (!kCached || look)
             {
                 best = 0ull;
-#pragma unroll 4
                 for (uint32_t i = lane; i < pool; i += 32)
                 {
                     const uint64_t record = records[i];
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(kRouteThreads) router_select_kernel(const Rout
     const uint32_t token_begin = blockIdx.x * a.tokens_per_block;
     const uint32_t token_end = min(a.token_count, token_begin + a.tokens_per_block);
     for (uint32_t token = token_begin + warp; token < token_end; token += kRouteWarps)
-        select_token(a, token, scores, records, radix_bins, block_counts, error_word, a.selected_expert + static_cast<size_t>(token) * top_k,
+        select_token<false>(a, token, scores, records, radix_bins, block_counts, error_word, a.selected_expert + static_cast<size_t>(token) * top_k,
                      a.selected_weight + static_cast<size_t>(token) * top_k);
     __syncthreads();
     // this block's column of the [expert][block] table
@@ -475,7 +476,8 @@ __global__ void __launch_bounds__(kRouteThreads) router_place_kernel(const Route
 // a contiguous run of tokens and keeps its routes and their counts in shared memory; after one cluster barrier it
 // reads its peers' counts, scans the totals into CSR offsets and places its own routes.
 // What bounds it: the latency of one token's selection (exp, k arg-max rounds) and of the launch; three launches with
-// a table in global memory between them cost 11.7 us for 32 tokens of 128 experts (7.7 here), 17.4 for 64 of 256 (11.6).
+// a table in global memory between them cost 11.8 us for 32 tokens of 128 experts, top 4 (6.7 here), 13.4 for 64 of 256,
+// top 8 (9.4).
 constexpr uint32_t kFewCtas = 8;
 constexpr uint32_t kFewThreads = 512;
 constexpr uint32_t kFewWarps = kFewThreads / 32;
@@ -519,7 +521,7 @@ __global__ void __cluster_dims__(kFewCtas, 1, 1) __launch_bounds__(kFewThreads) 
     const uint32_t token_begin = min(a.token_count, rank * per);
     const uint32_t token_end = min(a.token_count, token_begin + per);
     for (uint32_t token = token_begin + warp; token < token_end; token += kFewWarps)
-        select_token(a, token, scores, records, nullptr, counts, &error_word, route_expert + (token - token_begin) * top_k,
+        select_token<true>(a, token, scores, records, nullptr, counts, &error_word, route_expert + (token - token_begin) * top_k,
                      route_weight + (token - token_begin) * top_k);
     cluster.sync();
 
@@ -657,10 +659,16 @@ __global__ void __launch_bounds__(256) regroup_gather_kernel(const float* hidden
     }
 }
 
-// Whether one launch serves the call.  It uses none of the scratch in RouterArgs.
+// Whether one launch serves the call.  It uses none of the scratch in RouterArgs.  Its eight SMs evaluate the scores of all
+// tokens in double precision: beyond 48 Ki sigmoids or softpluses the three launches over all SMs are faster.  One against
+// three launches, us, 128 tokens, top 16, sqrt-softplus: 384 experts 24.6 against 24.6, 512 30.6 against 27.3, 1024 53 against
+// 41.5 (sigmoid 19.4 against 20.5, 23.8 against 21.7, 39.6 against 30.5).  Softmax rows are bound by the sum in index order
+// instead: 128 tokens, top 16, 768 experts 34.4 against 36.5, 1024 46.1 against 44.5.
 bool in_one_launch(uint32_t token_count, const moe_router_options& options)
 {
-    return token_count <= kFewTokens && options.expert_count <= kNarrowExperts && options.top_k <= kNarrowTopK;
+    const uint32_t most_scores = (options.score_function == MOE_ROUTER_SOFTMAX ? 96u : 48u) * 1024u;
+    return token_count <= kFewTokens && options.expert_count <= kNarrowExperts && options.top_k <= kNarrowTopK &&
+           token_count * options.expert_count <= most_scores;
 }
 
 } // namespace

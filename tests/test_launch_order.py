@@ -123,16 +123,17 @@ class Captured:
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("tokens,experts,top_k,launches", [(32, 128, 4, 1), (128, 1024, 16, 1), (129, 64, 4, 4), (4, 1025, 2, 4), (4, 64, 17, 4)])
-def test_static_router_launches_what_it_needs(pkg, sampler, torch_cuda, tokens, experts, top_k, launches):
+@pytest.mark.parametrize("tokens,experts,top_k,score,launches", [(32, 128, 4, 0, 1), (128, 768, 16, 0, 1), (128, 1024, 16, 0, 4), (129, 64, 4, 0, 4), (4, 1025, 2, 0, 4), (4, 64, 17, 0, 4),
+                                                                 (128, 384, 8, 1, 1), (128, 385, 8, 1, 4), (128, 384, 8, 2, 1), (49, 1004, 8, 2, 4)])
+def test_static_router_launches_what_it_needs(pkg, sampler, torch_cuda, tokens, experts, top_k, score, launches):
     """One launch for a few tokens; the three launches over the fixed scratch follow a reset of its counters."""
     torch = torch_cuda
     generator = torch.Generator(device="cuda").manual_seed(tokens)
     logits = torch.randn((tokens, experts), generator=generator, device="cuda")
-    want = sampler.router_dispatch(logits, top_k)
+    want = sampler.router_dispatch(logits, top_k, score_function=score)
     torch.cuda.synchronize()
     got = pkg.DispatchPlan(*[torch.empty_like(t) for t in (want.expert_offsets, want.route_token, want.route_rank, want.route_weight, want.status)])
-    options = pkg.RouterOptions(experts, top_k, pkg.ROUTER_SOFTMAX, 1, 1.0, pkg.ROUTER_FLAG_NORMALIZE_TOPK, None, None)
+    options = pkg.RouterOptions(experts, top_k, score, 1, 1.0, pkg.ROUTER_FLAG_NORMALIZE_TOPK, None, None)
 
     def dispatch(stream):
         message = C.create_string_buffer(256)
