@@ -319,6 +319,15 @@ def fresh_outputs(torch, rows):
             "flags": torch.empty(rows, dtype=torch.int32, device="cuda"), "status": torch.empty(rows, dtype=torch.int32, device="cuda"), "topk": None}
 
 
+def kernels_per_call(package, params, dtype_label):
+    """Kernels one sample_batch call launches: the streaming kernel; behind it the one-CTA exact kernel when a row has no Top-K or
+    one above its limit, and before that the clusters when fp32 rows have none."""
+    drawn = params["temperature"] > 0
+    untruncated = bool(np.any(drawn & (params["top_k"] == 0)))
+    exact = untruncated or bool(np.any(drawn & (params["top_k"] > package.TOPK_FAST_MAX)))
+    return 1 + int(exact) + int(untruncated and dtype_label == "f32")
+
+
 def oracle_tokens(oracle, package, logits, params, step_offset, rows, threads):
     uniforms = np.array([package.philox_uniform(p["seed"], p["row_id"], int(p["step"]) + step_offset) for p in params[:rows]], dtype=np.float32)
     return oracle.sample_batch(logits[:rows], params["temperature"][:rows], params["top_k"][:rows], params["top_p"][:rows],
@@ -493,8 +502,8 @@ def run_speculative_bench(args, as_dict=False):
     line = {"metric": "speculative verifications/s, 4 proposed tokens, vocab 201088", "value": 1e3 / ms, "unit": "verifications/s", "n_gpus": 1,
             "steps": steps, "warmup": max(args.warmup, 3), "ms_per_step": ms, "higher_is_better": True, "dtype": "f32", "data": "synthetic",
             "config": {"workload": "5 target + 4 draft rows x 201088 fp32 2.5*N(0,1) (draft = target + noise), T=1 top_k=40 top_p=0.95; direct C-ABI calls, "
-                                   "device-resident logits, 4 cases rotated", "kernels_per_step": 3, "bytes_read_per_step": 9 * vocab * 4},
-            "gpu_launches": 3 * steps,
+                                   "device-resident logits, 4 cases rotated", "kernels_per_step": 2, "bytes_read_per_step": 9 * vocab * 4},
+            "gpu_launches": 2 * steps,
             "cpu_baseline": {"value": len(cases) / t_cpu, "unit": "verifications/s", "cores": 1, "kind": oracle.kind,
                              "sample": f"{len(cases)} verifications, single thread (a Session verifies on its own thread)"},
             "results_equal_to_reference": f"{equal}/{len(cases)}",
@@ -535,13 +544,12 @@ def side_workload(torch, package, workloads, oracle, name, steps, peak, threads)
     rotation = 4 if bytes_per_step * 4 <= 8 << 30 else 2
     batches = [device] + [device.roll(shift, 0).contiguous() for shift in range(1, rotation)]
     timing = time_sampler_workload(torch, package, sampler, batches, params, steps, 0.15)
-    needs_exact = bool(np.any((params["temperature"] > 0) & ((params["top_k"] == 0) | (params["top_k"] > package.TOPK_FAST_MAX))))
     entry = {"workload": description + (f"; timed on {timed_rows} rows ({rows} distinct rows tiled)" if timed_rows != rows else ""), "dtype": dtype_label,
              "ms_per_step": timing["overlapped"]["ms_per_step"], "ms_per_step_single_launch": timing["single_launch"]["ms_per_step"],
              "rows_per_s": timed_rows / (timing["overlapped"]["ms_per_step"] * 1e-3),
              "frac": bytes_per_step / (timing["overlapped"]["ms_per_step"] * 1e-3) / 1e9 / peak,
              "frac_single_launch": bytes_per_step / (timing["single_launch"]["ms_per_step"] * 1e-3) / 1e9 / peak,
-             "kernels_per_step": 2 if needs_exact else 1,
+             "kernels_per_step": kernels_per_call(package, params, dtype_label),
              "token_ids_equal": f"{agree}/{rows}", "oracle": oracle.kind}
     sampler.close()
     del batches, device
@@ -757,8 +765,7 @@ def main() -> int:
     batches = [base] + [base[torch.from_numpy(p).cuda()].contiguous() for p in permutations[1:]]
     first = sampler.sample_batch(batches[0], params)  # uploads the per-row parameters once; later calls reuse them
     torch.cuda.synchronize()
-    needs_exact = bool(np.any((params["temperature"] > 0) & ((params["top_k"] == 0) | (params["top_k"] > package.TOPK_FAST_MAX))))
-    launches_per_step = 2 if needs_exact else 1
+    launches_per_step = kernels_per_call(package, params, dtype_label)
 
     # every step of a graph writes its own output buffers, so that tokens produced inside the
     # timed region can be checked afterwards

@@ -92,12 +92,12 @@ typedef struct moe_sampler moe_sampler;
  * reference sampler is stateless apart from Session::random_generator_). */
 int moe_sampler_create(int device, uint32_t max_rows, uint32_t max_vocab, moe_sampler** out);
 void moe_sampler_destroy(moe_sampler* sampler);
-/* Back-to-back sampling calls on one stream normally run one after the other.
- * With overlap enabled, moe_sample_batch launches its kernel with programmatic
- * stream serialization: its CTAs may take the SM slots the previous sampling
- * kernel of the stream leaves free and read their logits while that kernel is
- * still running, and they wait for it to complete before they write anything.
- * Results are unchanged.  Enable it only when the logits of a call do not
+/* Back-to-back sampling calls on one stream normally run one after the other:
+ * a kernel may be placed on free SMs early, but waits for the kernel before it
+ * before it reads or writes anything.  With overlap enabled, the CTAs of
+ * moe_sample_batch read their logits while the previous sampling kernel of the
+ * stream is still running, and wait for it to complete before they write
+ * anything.  Results are unchanged.  Enable it only when the logits of a call do not
  * depend on the kernel launched immediately before it on the same stream
  * (independent batches, or logits produced earlier): that kernel is not waited
  * for before the logits are read.  Off by default.  No reference counterpart

@@ -21,7 +21,7 @@
 // byte digits, match.any aggregation, six passes over L2 and a bitonic sort in
 // shared memory, before and after: 64 rows x 40000 scores, top 2048 82.0 -> 27.3 us;
 // 64 x 131072, top 2048 260 -> 72; 64 x 2300, top 2048 30.0 -> 11.4; 1000 x 2300, top
-// 512 75.7 -> 50.7; 64 x 1024, top 512 13.3 -> 6.6; 4000 x 300, top 64 130 -> 59.  What
+// 512 75.7 -> 50.7; 64 x 1024, top 512 13.3 -> 6.6; 4000 x 300, top 64 130 -> 55.  What
 // got slower: rows between 1024 and some 9000 scores that nearly all agree in the upper
 // 14 key bits take all three digits and the network (1000 x 2300, top 512, 1 + 1e-6 N(0,1)
 // 76.8 -> 87.3; 64 of them 16.8 -> 16.6; top 64 12.7 -> 15.7).

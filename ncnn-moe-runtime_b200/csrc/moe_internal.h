@@ -102,9 +102,9 @@ struct SampleArgs
     // some row has a Top-K too large for the small record buffer: use the
     // large-buffer instantiation (fewer CTAs per SM)
     bool large_top_k;
-    // launched with programmatic stream serialization: the kernel may start
-    // while the previous kernel of the stream is still finishing, so it waits
-    // for that kernel (griddepcontrol.wait) before its first global write
+    // moe_sampler_set_overlap: the streaming kernel reads its parameters and logits while the kernel before it is still
+    // running and waits for that kernel (griddepcontrol.wait) before it touches anything else; without it the wait is
+    // the first thing it does
     bool overlap_previous;
     // the exact kernels follow in the same call and may take their places on the SMs while this one runs
     bool release_exact;
@@ -268,9 +268,11 @@ ClusterOccupancy cluster_occupancy(ClusterOccupancyTable& table, int device, Que
     return found;
 }
 
-// Kernels are launched while the kernel before them in the stream may still run (programmatic stream serialization)
-// and wait for it before they touch memory (wait_for_previous_kernel): the launch itself is out of the way when the
-// earlier kernel ends.  1 to 3 us per launch here.
+// All kernels but the router's three launches (and the reset before them in moe_router_dispatch_static) are launched while
+// the kernel before them in the stream may still run (programmatic stream serialization) and wait for it before they
+// touch memory (wait_for_previous_kernel): the launch itself is out of the way when the earlier kernel ends.
+// 1 to 3 us per launch.  The loads behind the wait are coherent ones: ld.global.nc and __ldg are for data that nobody
+// writes while the kernel is resident.
 inline cudaLaunchAttribute follow_closely()
 {
     cudaLaunchAttribute attribute = {};

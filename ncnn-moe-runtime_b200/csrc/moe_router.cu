@@ -591,8 +591,8 @@ __global__ void __cluster_dims__(kFewCtas, 1, 1) __launch_bounds__(kFewThreads) 
 // One warp per piece of a route's row: 4 KiB (eight 16-byte loads in flight per lane, whole 128-byte lines), so that
 // a decode step's few rows spread over the SMs too; whole rows in calls that write more than L2 holds.
 // What bounds it: HBM writes; the hidden rows are read once per route of their token and stay in L2.  32768 rows of
-// 16 KiB: 126 us, 4.8 TB/s (bulk copies through shared memory: 135 us, and 39 against 24 us for rows of 4 KiB).
-// 128 rows of 11.25 KiB: 6.7 -> 5.4 us with pieces.
+// 16 KiB: 121 us, 5.0 TB/s (bulk copies through shared memory took 135 us against 126 then, and 39 against 24 us for rows of
+// 4 KiB).  128 rows of 11.25 KiB, back to back: 4.3 us with whole rows, 2.8 with pieces.
 constexpr uint32_t kGatherPiece = 8u * 32u; // 16-byte vectors
 
 __global__ void __launch_bounds__(256) regroup_gather_kernel(const float* hidden, uint32_t token_count, uint32_t columns, const uint32_t* route_token,
