@@ -67,6 +67,7 @@ constexpr uint32_t kHead = 192;          // candidates added literally, rounded 
 constexpr uint32_t kHeadCapacity = 512;
 constexpr uint32_t kLiteralGroups = 96;
 constexpr uint32_t kLiteralItems = 3072; // dense rows (90 items a group) mark up to thirty groups that refining does not spare
+constexpr uint32_t kFewLiteralItems = 256;
 constexpr uint32_t kMaxCluster = 16;
 constexpr uint32_t kDeadGroup = 0xFFFFu;
 constexpr int kGuardUnits = 64;          // a group this close to the end of a binade or to the bound is literal
@@ -126,8 +127,8 @@ struct alignas(16) ClusterShared
     uint64_t head_in[kHeadCapacity];
     uint64_t head[kHeadCapacity];
     float head_value[kHeadCapacity];
-    uint64_t item[kLiteralItems];          // as they come, and in rank order
-    uint64_t item_by_group[kLiteralItems]; // in between: group by group
+    uint64_t item[kLiteralItems];          // as they come; many of them in rank order too
+    uint64_t item_by_group[kLiteralItems]; // many: group by group; few: in rank order
     float item_value[kLiteralItems];
     LiteralGroup literal_in[kLiteralGroups];
     LiteralGroup literal[kLiteralGroups];
@@ -1054,6 +1055,12 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                         cs.literal_begin[before] = items_before;
                         cs.literal_end[before] = items_before; // grows to the end as the items come in
                     }
+                    // Rank order: a few items are compared all with all; more of them inside their groups, behind two more
+                    // barriers (half a microsecond), where all with all grows to 180 us for a dense row's 2400.
+                    const bool few = items <= kFewLiteralItems;
+                    const uint64_t* const ranked = few ? cs.item_by_group : cs.item;
+                    if (few)
+                        rank_records(cs.item, cs.item_by_group, items);
                     __syncthreads();
                     // place in `literal` of an item's group
                     const auto literal_of = [&](uint64_t record) {
@@ -1069,27 +1076,29 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                         }
                         return low;
                     };
-                    for (uint32_t i = tid; i < items; i += kExactThreads)
+                    if (!few)
                     {
-                        const uint64_t record = cs.item[i];
-                        cs.item_by_group[atomicAdd(&cs.literal_end[literal_of(record)], 1u)] = record;
-                    }
-                    __syncthreads();
-                    // a group's items by their rank among themselves: comparing every two items of a dense row's 2400 took 180 us
-                    for (uint32_t i = tid; i < items; i += kExactThreads)
-                    {
-                        const uint64_t record = cs.item_by_group[i];
-                        const uint32_t at = literal_of(record);
-                        uint32_t rank_in_group = 0;
+                        for (uint32_t i = tid; i < items; i += kExactThreads)
+                        {
+                            const uint64_t record = cs.item[i];
+                            cs.item_by_group[atomicAdd(&cs.literal_end[literal_of(record)], 1u)] = record;
+                        }
+                        __syncthreads();
+                        for (uint32_t i = tid; i < items; i += kExactThreads)
+                        {
+                            const uint64_t record = cs.item_by_group[i];
+                            const uint32_t at = literal_of(record);
+                            uint32_t rank_in_group = 0;
 #pragma unroll 4
-                        for (uint32_t j = cs.literal_begin[at]; j < cs.literal_end[at]; ++j)
-                            rank_in_group += cs.item_by_group[j] > record ? 1u : 0u;
-                        cs.item[cs.literal_begin[at] + rank_in_group] = record;
+                            for (uint32_t j = cs.literal_begin[at]; j < cs.literal_end[at]; ++j)
+                                rank_in_group += cs.item_by_group[j] > record ? 1u : 0u;
+                            cs.item[cs.literal_begin[at] + rank_in_group] = record;
+                        }
+                        __syncthreads();
                     }
-                    __syncthreads();
                     for (uint32_t i = tid; i < items; i += kExactThreads)
                     {
-                        const uint64_t record = cs.item[i];
+                        const uint64_t record = ranked[i];
                         float value = exact_expf(scaled_offset(key_to_float(record_key(record)), p.temperature, peak));
                         bool listed = true;
                         if (sum >= 1)
@@ -1128,7 +1137,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                         else if (sum == 1)
                         {
                             state.kept_total = walk.acc;
-                            state.threshold = walk.stopped ? cs.item[walk.item] : 0ull;
+                            state.threshold = walk.stopped ? ranked[walk.item] : 0ull;
                         }
                         else
                         {
@@ -1136,7 +1145,7 @@ __device__ __noinline__ bool exact_row_cluster(const SampleArgs& a, uint32_t row
                             state.action = kActionDone;
                             uint64_t chosen = 0;
                             if (walk.stopped)
-                                chosen = cs.item[walk.item];
+                                chosen = ranked[walk.item];
                             else if (threshold != 0)
                                 chosen = threshold; // session.cpp:441-442: the last candidate if the sum never passes the uniform
                             else
