@@ -60,7 +60,7 @@ constexpr uint32_t kGroups = 16384;
 // unless the unit was guessed far too small, and kGroupLimit such steps fit the 31 bits of a counter.  The limit ends in
 // one half, so that an item that reaches it looks like a tie and makes its group literal.
 // With 120 items per group rows with 267 equal logits were left after two passes: 8 of them took 629 us, 604 without
-// the clusters, 138 now; 256 of them 2690, 2280 and 765.
+// the clusters, 138 now; 256 of them 2690, 2280 and 730.
 constexpr uint32_t kGroupLimit = 3072;
 constexpr float kStepLimit = 131071.5f;
 constexpr uint32_t kHead = 192;          // candidates added literally, rounded up to whole groups
